@@ -977,7 +977,8 @@ def main():
                         layout=layout)
     # the layout the library runs (hs_config.layout 0 chooses by image size)
     wide = (not args.exact) and (layout == 2 or (layout == 0 and H * W >= 2_000_000))
-    passes = (iters + T - 1) // T
+    # T = 0: the library holds the image on the chip for all sweeps (one launch)
+    passes = (iters + T - 1) // T if T else 1
     flush = torch.empty(L2_FLUSH_BYTES // 4, dtype=torch.float32, device="cuda")
 
     uv = D.empty_planes(2, H, W)
@@ -1096,7 +1097,7 @@ def main():
     big = H * W >= 3000000
     kernel = (f"hs_stream_w_kernel<{T},{'true' if big else 'false'}>" if wide else
               f"hs_stream_kernel<{T},{'false' if args.exact else 'true'},"
-              f"{'true' if T <= 2 else 'false'}>")
+              f"{'true' if T <= 2 else 'false'}>") if T else "hs_resident_kernel"
     # ncu figures of this very kernel at this shape (profiles/), when one was captured
     traffic, prof = None, {}
     tpath = os.path.join(HERE, "profiles", "sweep_traffic.json")

@@ -91,8 +91,9 @@ def best_sweep_config(H: int, W: int, ld: int, fast_math: bool = True,
                       candidates=T_CANDIDATES,
                       sweeps: int = DEFAULT_TUNING_SWEEPS) -> Tuple[int, int, int]:
     """(sweeps_per_pass, rows_per_segment, layout) fastest on the current device for HxW;
-    both layouts (2 and 4 columns per lane) compete in the fast form.  Every candidate is timed
-    over `sweeps` sweeps: pass the workload's own count when it is known (the last, partial
+    both layouts (2 and 4 columns per lane) compete in the fast form, and (0, 0, 0), the
+    library's own choice, which holds an image that fits the chip there for all sweeps.  Every
+    candidate is timed over `sweeps` sweeps: pass the workload's own count when it is known (the last, partial
     pass differs by depth)."""
     import torch
 
@@ -119,6 +120,7 @@ def best_sweep_config(H: int, W: int, ld: int, fast_math: bool = True,
             for seg in _seg_candidates(H, W, T):
                 ms = time_config(Ix, Iy, It, u, v, T, seg, fast_math, sweeps, layout=layout)
                 results.append((ms, T, seg, layout))
+    results.append((time_config(Ix, Iy, It, u, v, 0, 0, fast_math, sweeps), 0, 0, 0))
     results.sort()
     best = tuple(results[0][1:])
     log = os.environ.get("HS_AUTOTUNE_LOG")

@@ -96,19 +96,11 @@ __device__ __forceinline__ float2 mul2r(float2 a, float2 b) {
 }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
-// Horn-Schunck 2x2x2 derivatives at (x, y).  Tap order (0,0) (1,0) (0,1) (1,1), taps
-// clamped to the image; each accumulator sums from 0 in that order, one rounding per
-// operation; then Ix = DxI0 + DxI1, Iy = DyI0 + DyI1, It = DtI1 - DtI0.
-__device__ __forceinline__ void hs_derivs_at(const float *__restrict__ I0,
-                                             const float *__restrict__ I1, int x, int y, int H,
-                                             int W, int ld, float &Ix, float &Iy, float &It) {
-    const int x1 = min(x + 1, W - 1);
-    const int y1 = min(y + 1, H - 1);
-    const size_t r0 = (size_t)y * ld, r1 = (size_t)y1 * ld;
-    const float a[4] = {__ldg(I0 + r0 + x), __ldg(I0 + r0 + x1), __ldg(I0 + r1 + x),
-                        __ldg(I0 + r1 + x1)};
-    const float b[4] = {__ldg(I1 + r0 + x), __ldg(I1 + r0 + x1), __ldg(I1 + r1 + x),
-                        __ldg(I1 + r1 + x1)};
+// Horn-Schunck 2x2x2 derivatives from the four taps (0,0) (1,0) (0,1) (1,1) of both images:
+// each accumulator sums from 0 in that order, one rounding per operation; then
+// Ix = DxI0 + DxI1, Iy = DyI0 + DyI1, It = DtI1 - DtI0.
+__device__ __forceinline__ void hs_derivs_taps(const float (&a)[4], const float (&b)[4], float &Ix, float &Iy,
+                                               float &It) {
     const float wx[4] = {-0.25f, 0.25f, -0.25f, 0.25f};
     const float wy[4] = {-0.25f, -0.25f, 0.25f, 0.25f};
     float ax0 = 0.f, ax1 = 0.f, ay0 = 0.f, ay1 = 0.f, at0 = 0.f, at1 = 0.f;
@@ -124,6 +116,20 @@ __device__ __forceinline__ void hs_derivs_at(const float *__restrict__ I0,
     Ix = __fadd_rn(ax0, ax1);
     Iy = __fadd_rn(ay0, ay1);
     It = __fsub_rn(at1, at0);
+}
+
+// The derivatives at (x, y), taps clamped to the image.
+__device__ __forceinline__ void hs_derivs_at(const float *__restrict__ I0,
+                                             const float *__restrict__ I1, int x, int y, int H,
+                                             int W, int ld, float &Ix, float &Iy, float &It) {
+    const int x1 = min(x + 1, W - 1);
+    const int y1 = min(y + 1, H - 1);
+    const size_t r0 = (size_t)y * ld, r1 = (size_t)y1 * ld;
+    const float a[4] = {__ldg(I0 + r0 + x), __ldg(I0 + r0 + x1), __ldg(I0 + r1 + x),
+                        __ldg(I0 + r1 + x1)};
+    const float b[4] = {__ldg(I1 + r0 + x), __ldg(I1 + r0 + x1), __ldg(I1 + r1 + x),
+                        __ldg(I1 + r1 + x1)};
+    hs_derivs_taps(a, b, Ix, Iy, It);
 }
 #endif
 

@@ -1,0 +1,341 @@
+// hs_resident.cuh -- the resident form of the Horn-Schunck sweeps: the whole image lives on
+// the chip for all sweeps of a call, one tile per CTA and one CTA per SM, in a cooperative
+// launch.
+//
+// The streaming kernels (hs_stream.cuh, hs_stream4.cuh) read and write every plane once per
+// pass of T sweeps, and near L2-resident sizes they spend about half of their instructions on
+// the temporal halo, the rings and the copies.  An image of up to about 2 Mpx fits the 148 SMs:
+//   - the state (u, v) of a tile of 128 columns x (NW * R) rows sits in registers, R rows of 4
+//     adjacent columns per lane (a warp owns R whole rows of the tile);
+//   - the four coefficients of each pixel (Ix, Iy, It and the negated denominator term) sit in
+//     tensor memory: 16 words per lane and row, 512 columns x 128 lanes for the largest tile.
+//     Every warp reads back only what it wrote; tcgen05.ld delivers about 900 B per clock and
+//     SM, where shared memory, which the shuffles also use, delivers 128;
+//   - within a sweep, horizontal neighbours come from warp shuffles, vertical ones from the
+//     lane's own rows; a warp publishes its first and last row's contribution to its two
+//     neighbour warps through shared memory (one block barrier per sweep);
+//   - every kResT sweeps the CTAs exchange a ring of kResT pixels around their tiles through
+//     global memory (L2); between exchanges a tile runs kResT sweeps on its own, the valid
+//     region shrinking into the kResT-pixel halo.
+// Every cell sees the operations of the streaming kernels in their order, so the results are
+// the same bit for bit, in both forms.
+//
+// Image sides.  The lane at column 0 and the lane at column W-1 substitute their own value for
+// the missing neighbour (two selects per row and plane, in the tiles at a side only).  Row -1
+// and row H are kept equal to rows 0 and H-1 (copied after every sweep), so no row of the sweep
+// itself is special.
+//
+// Exchange.  The warps put their ring into shared memory, then all threads of the CTA send and
+// receive it together, three messages each, and the halo goes back through shared memory: one
+// round trip to L2 per exchange.  (Each warp receiving its own halo took a round trip per
+// message in the warps that hold halo rows: 14000 clocks per exchange at 1080p.)  A message is
+// 16 bytes, three state values and the exchange's number, stored and loaded as one 128-bit
+// access: a reader polls the message itself until it carries the number it waits for, so no
+// flag and no fence stands between the store and the load.  Exchange e = 1, 2, ... uses half
+// e % 2 of a tile's outbox.  A tile writes a half again at e + 2, after it has received e + 1
+// from all its neighbours, which they sent after a block barrier behind their reads of e.  The
+// outboxes are cleared before the launch (numbers start at 1).  Every wait is bounded
+// (hs_resident.cu).
+#pragma once
+
+#include "hs_stream.cuh"
+
+namespace hs {
+
+constexpr int kResT = 4;                      // sweeps between exchanges = halo pixels
+constexpr int kResCols = 128;                 // columns of a tile, halo included (4 per lane)
+constexpr int kResChunks = kResCols / 4 - 2;  // 4-column chunks of a tile's own region, at most
+
+struct ResidentParams {
+    const float *I0, *I1;        // if set: the images; the kernel forms the derivatives itself
+    const float *Ix, *Iy, *It;   // else the derivative planes
+    float *u, *v;                // state: read at the start (unless zero_start), written at the end
+    float4 *box;                 // outboxes of all tiles, then one word: the abort flag
+    unsigned *abort_flag;
+    int H, W, ld;
+    float alpha2;
+    float we, wc;
+    int ntx, nty;                // tiles across and down
+    int iters, nblocks;          // the sweeps run in nblocks blocks of at most kResT
+    int zero_start;
+};
+
+// The chunks (4 pixels of u and of v, 8 floats) a tile sends and receives in one exchange:
+//   row blocks    [up, down][kResT rows][32 lanes]  sent: its first / last kResT own rows;
+//                                                   received: the rows above / below them
+//   column blocks [left, right][rows of the tile]   its first / last own chunk of every row;
+//                                                   the chunks beside them
+// A chunk is three messages: message m holds floats 3m .. 3m+2 and the exchange's number.
+constexpr int kResRowChunks = kResT * 32;
+__host__ __device__ constexpr int res_chunks(int rows) { return 2 * kResRowChunks + 2 * rows; }
+__host__ __device__ constexpr int res_msgs(int rows) { return 3 * res_chunks(rows); }
+
+// first pixel row of tile row j of n over H rows; first 4-column chunk likewise
+__host__ __device__ inline int res_split(int j, int n, int total) {
+    return (int)((long long)j * total / n);
+}
+
+// ---- tensor memory as per-warp storage (32 lanes x 32-bit columns; warp w of a CTA reaches
+// lanes 32 (w % 4) .. + 31)
+
+__device__ __forceinline__ void tmem_st16(unsigned addr, const float (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"f"(r[0]), "f"(r[1]), "f"(r[2]),
+        "f"(r[3]), "f"(r[4]), "f"(r[5]), "f"(r[6]), "f"(r[7]), "f"(r[8]), "f"(r[9]), "f"(r[10]),
+        "f"(r[11]), "f"(r[12]), "f"(r[13]), "f"(r[14]), "f"(r[15]), "r"(addr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(float (&r)[16], unsigned addr) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]),
+          "=f"(r[8]), "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15])
+        : "r"(addr));
+}
+// The loaded registers hold their values after this wait; they pass through it as operands so
+// that no use of them can be scheduled before it.
+__device__ __forceinline__ void tmem_wait_ld(float (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]), "+f"(r[4]), "+f"(r[5]), "+f"(r[6]),
+                   "+f"(r[7]), "+f"(r[8]), "+f"(r[9]), "+f"(r[10]), "+f"(r[11]), "+f"(r[12]), "+f"(r[13]),
+                   "+f"(r[14]), "+f"(r[15]));
+}
+__device__ __forceinline__ void tmem_wait_st() {
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ float2 lo2(float4 a) { return make_float2(a.x, a.y); }
+__device__ __forceinline__ float2 hi2(float4 a) { return make_float2(a.z, a.w); }
+__device__ __forceinline__ float4 cat4(float2 a, float2 b) { return make_float4(a.x, a.y, b.x, b.y); }
+
+// Per-lane constants of a tile.
+struct ResLane {
+    int lane, warp;
+    bool first, last;  // the lane holds column 0 / column W-1
+    int row0;          // image row of the warp's first row
+    int H;
+    unsigned tmem;     // the warp's tensor memory
+};
+
+// Left and right neighbours of a lane's 4 columns (E, O) = ((c0, c1), (c2, c3)) across the
+// warp.  SIDE: -1 = no image side in the tile; else the lane column (0..3) that W-1 falls on.
+template <int SIDE>
+__device__ __forceinline__ void res_neighbours(const ResLane &t, float2 E, float2 O, float2 &lE, float2 &rE,
+                                               float2 &lO, float2 &rO) {
+    const float lsh = __shfl_up_sync(kFull, O.y, 1);
+    const float rsh = __shfl_down_sync(kFull, E.x, 1);
+    float L0 = lsh, R0 = E.y, R1 = O.x, R2 = O.y, R3 = rsh;
+    if constexpr (SIDE >= 0) L0 = t.first ? E.x : L0;
+    if constexpr (SIDE == 0) R0 = t.last ? E.x : R0;
+    if constexpr (SIDE == 1) R1 = t.last ? E.y : R1;
+    if constexpr (SIDE == 2) R2 = t.last ? O.x : R2;
+    if constexpr (SIDE == 3) R3 = t.last ? O.y : R3;
+    lE = make_float2(L0, E.x);
+    rE = make_float2(R0, R1);
+    lO = make_float2(E.y, O.x);
+    rO = make_float2(R2, R3);
+}
+
+// What a row contributes to the rows around it, for one plane and column pair.
+//   fast : h = left + right and Y = we c + wc h (the row's term as an upper or lower row)
+//   exact: the five products of the taps and the running sum `up` of the three upper taps
+template <bool FAST>
+struct RowTerm;
+template <>
+struct RowTerm<true> {
+    float2 h, Y;
+};
+template <>
+struct RowTerm<false> {
+    float2 tl, tc, tr, ml, mr, up;
+};
+
+template <int SIDE>
+__device__ __forceinline__ void row_terms(const ResLane &t, float2 E, float2 O, float2 we, float2 wc,
+                                          RowTerm<true> (&o)[2]) {
+    float2 lE, rE, lO, rO;
+    res_neighbours<SIDE>(t, E, O, lE, rE, lO, rO);
+    o[0].h = make_float2(__fadd_rn(lE.x, rE.x), __fadd_rn(lE.y, rE.y));
+    o[1].h = make_float2(__fadd_rn(lO.x, rO.x), __fadd_rn(lO.y, rO.y));
+    o[0].Y = fma2(we, E, mul2(wc, o[0].h));
+    o[1].Y = fma2(we, O, mul2(wc, o[1].h));
+}
+template <int SIDE>
+__device__ __forceinline__ void row_terms(const ResLane &t, float2 E, float2 O, float2 we, float2 wc,
+                                          RowTerm<false> (&o)[2]) {
+    float2 l[2], r[2];
+    res_neighbours<SIDE>(t, E, O, l[0], r[0], l[1], r[1]);
+    const float2 c[2] = {E, O};
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        o[j].tl = mul2r(wc, l[j]);
+        o[j].tc = mul2r(we, c[j]);
+        o[j].tr = mul2r(wc, r[j]);
+        o[j].ml = mul2r(we, l[j]);
+        o[j].mr = mul2r(we, r[j]);
+        o[j].up = add2(add2(add2(f2(0.f, 0.f), o[j].tl), o[j].tc), o[j].tr);
+    }
+}
+
+// Jacobi update of a column pair from its averages; (cx, cy, ct, nd) as in the streaming
+// kernels: nd = -1/den (fast) or -den (exact).
+template <bool FAST>
+__device__ __forceinline__ void res_update(float2 ubar, float2 vbar, float2 cx, float2 cy, float2 ct, float2 nd,
+                                           float2 &u, float2 &v) {
+    if constexpr (FAST) {
+        const float2 nt = mul2(fma2(cx, ubar, fma2(cy, vbar, ct)), nd);
+        u = fma2(cx, nt, ubar);
+        v = fma2(cy, nt, vbar);
+    } else {
+        const float2 r = add2(add2(mul2r(cx, ubar), mul2r(cy, vbar)), ct);
+        const float2 nt = f2(__fdiv_rn(r.x, nd.x), __fdiv_rn(r.y, nd.y));
+        u = add2(ubar, mul2r(cx, nt));
+        v = add2(vbar, mul2r(cy, nt));
+    }
+}
+
+// The block barrier of a sweep.  Warps reach it from different variants of res_sweep (image
+// sides and edges), so it is the named-barrier instruction itself: it counts warps, not places.
+__device__ __forceinline__ void res_barrier() { asm volatile("bar.sync 0;" ::: "memory"); }
+
+// One sweep of the warp's R rows.  pub: this sweep's half of the publication buffer,
+// [NW][4][32] float4 (first row's u, v terms, last row's u, v terms).
+//   fast : the first and the last row's Y
+//   exact: the first row itself (its three lower taps are added one by one) and the last
+//          row's `up`
+template <bool FAST, int NW, int R, int SIDE>
+__device__ __forceinline__ void res_sweep(const ResLane &t, float2 (&cu)[R][2][2], float4 *pub, float wef,
+                                          float wcf) {
+    const float2 we = f2(wef, wef), wc = f2(wcf, wcf);
+    RowTerm<FAST> cur[2][2];  // [plane][pair]: terms of the row being finished
+    RowTerm<FAST> lst[2][2];  // of the last row
+    float4 *mine = pub + t.warp * 128 + t.lane;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        row_terms<SIDE>(t, cu[0][q][0], cu[0][q][1], we, wc, cur[q]);
+        if constexpr (R > 1) row_terms<SIDE>(t, cu[R - 1][q][0], cu[R - 1][q][1], we, wc, lst[q]);
+        else { lst[q][0] = cur[q][0]; lst[q][1] = cur[q][1]; }
+        if constexpr (FAST) {
+            mine[32 * q] = cat4(cur[q][0].Y, cur[q][1].Y);
+            mine[64 + 32 * q] = cat4(lst[q][0].Y, lst[q][1].Y);
+        } else {
+            mine[32 * q] = cat4(cu[0][q][0], cu[0][q][1]);
+            mine[64 + 32 * q] = cat4(lst[q][0].up, lst[q][1].up);
+        }
+    }
+    res_barrier();
+    // the tile's outermost rows have no neighbour warp: any value, they are halo (or outside)
+    const float4 *above = pub + max(t.warp - 1, 0) * 128 + 64 + t.lane;
+    const float4 *below = pub + min(t.warp + 1, NW - 1) * 128 + t.lane;
+    // row 0 as the warp's first row has itself above it, row H-1 as its last row itself below
+    const bool top = t.row0 == 0, bottom = t.row0 + R == t.H;
+
+    float2 acc[2][2];  // fast: Z = Y(r-1) + we h(r); exact: upper and middle taps of row r
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const float4 a4 = above[32 * q];
+        const float2 a[2] = {lo2(a4), hi2(a4)};
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            if constexpr (FAST) {
+                const float2 up = top ? cur[q][j].Y : a[j];
+                acc[q][j] = fma2(we, cur[q][j].h, up);
+            } else {
+                const float2 up = top ? cur[q][j].up : a[j];
+                acc[q][j] = add2(add2(up, cur[q][j].ml), cur[q][j].mr);
+            }
+        }
+    }
+    float co[16];
+    tmem_ld16(co, t.tmem);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        // terms of row r + 1
+        RowTerm<FAST> nxt[2][2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if (r + 1 < R - 1) {
+                row_terms<SIDE>(t, cu[r + 1 < R ? r + 1 : 0][q][0], cu[r + 1 < R ? r + 1 : 0][q][1], we, wc, nxt[q]);
+            } else if (r + 1 == R - 1) {
+                nxt[q][0] = lst[q][0];
+                nxt[q][1] = lst[q][1];
+            } else {  // the row below the warp's last row
+                const float4 b4 = below[32 * q];
+                if constexpr (FAST) {
+                    nxt[q][0].Y = bottom ? cur[q][0].Y : lo2(b4);
+                    nxt[q][1].Y = bottom ? cur[q][1].Y : hi2(b4);
+                } else {
+                    const float2 b0 = bottom ? cu[r][q][0] : lo2(b4), b1 = bottom ? cu[r][q][1] : hi2(b4);
+                    row_terms<SIDE>(t, b0, b1, we, wc, nxt[q]);
+                }
+            }
+        }
+        float2 avg[2][2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                if constexpr (FAST) {
+                    avg[q][j] = add2(acc[q][j], nxt[q][j].Y);
+                    if (r + 1 < R) acc[q][j] = fma2(we, nxt[q][j].h, cur[q][j].Y);
+                } else {
+                    avg[q][j] = add2(add2(add2(acc[q][j], nxt[q][j].tl), nxt[q][j].tc), nxt[q][j].tr);
+                    if (r + 1 < R) acc[q][j] = add2(add2(cur[q][j].up, nxt[q][j].ml), nxt[q][j].mr);
+                }
+            }
+        tmem_wait_ld(co);
+        float cn[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) cn[i] = co[i];
+        if (r + 1 < R) tmem_ld16(co, t.tmem + 16 * (r + 1));
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            res_update<FAST>(avg[0][j], avg[1][j], f2(cn[2 * j], cn[2 * j + 1]), f2(cn[4 + 2 * j], cn[5 + 2 * j]),
+                             f2(cn[8 + 2 * j], cn[9 + 2 * j]), f2(cn[12 + 2 * j], cn[13 + 2 * j]), cu[r][0][j],
+                             cu[r][1][j]);
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) cur[q][j] = nxt[q][j];
+    }
+}
+
+// The ghost rows: row -1 follows row 0 and row H row H-1, where both lie in this warp.  (Row 0
+// as a warp's first row and row H-1 as its last one are handled in the sweep.)
+template <int R>
+__device__ __forceinline__ void res_ghost_rows(const ResLane &t, float2 (&cu)[R][2][2]) {
+#pragma unroll
+    for (int r = 0; r + 1 < R; ++r) {
+        if (t.row0 + r == -1) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                cu[r][q][0] = cu[r + 1][q][0];
+                cu[r][q][1] = cu[r + 1][q][1];
+            }
+        }
+        if (t.row0 + r == t.H - 1) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                cu[r + 1][q][0] = cu[r][q][0];
+                cu[r + 1][q][1] = cu[r][q][1];
+            }
+        }
+    }
+}
+
+// n sweeps of the warp's rows; pub: both halves of the publication buffer, `half` the one to use.
+// (The loop is inside the variant: its state registers need not agree with another variant's
+// after every sweep.)
+template <bool FAST, int NW, int R, int SIDE>
+__device__ __forceinline__ void res_sweeps(const ResLane &t, float2 (&cu)[R][2][2], float4 *pub, int half, int n,
+                                           bool ghosts, float wef, float wcf) {
+#pragma unroll 1
+    for (int i = 0; i < n; ++i, half ^= 1) {
+        if (ghosts) res_ghost_rows<R>(t, cu);
+        res_sweep<FAST, NW, R, SIDE>(t, cu, pub + half * (NW * 128), wef, wcf);
+    }
+}
+
+}  // namespace hs

@@ -417,6 +417,24 @@ hs_status launch_pass(int T, bool fast, const SweepParams &pp, cudaStream_t s);
 hs_status run_passes_dev(const float *Ix, const float *Iy, const float *It, int H, int W, int ld,
                          float alpha2, const float *alpha_dev, int iters, float *u0, float *v0,
                          float *u1, float *v1, const ResolvedConfig &rc, cudaStream_t stream);
+
+// The resident form (hs_resident.cu): the tiling of an image that fits the chip.
+struct ResidentPlan {
+    int nw, r;         // warps per CTA and rows per warp
+    int ntx, nty;      // tiles across and down
+    int nblocks;       // blocks of sweeps between exchanges
+    size_t box_bytes;  // scratch for the exchanges
+};
+// false when the image does not fit (or the call is too short, or the scratch too small): the
+// streaming passes run it
+bool resident_plan(int H, int W, int iters, size_t scratch_bytes, ResidentPlan &pl);
+// `iters` sweeps on (u, v) in place, from zero when zero_start, on the given derivatives or,
+// when I0 is set, on those of the images.  scratch: box_bytes, 16-byte aligned.
+// HS_ERR_UNSUPPORTED, with no kernel launched, when the SMs at hand cannot hold the tiles all at
+// once.
+hs_status run_resident(const float *I0, const float *I1, const float *Ix, const float *Iy, const float *It, int H,
+                       int W, int ld, float alpha2, int iters, float *u, float *v, void *scratch, bool zero_start,
+                       const ResolvedConfig &rc, const ResidentPlan &pl, cudaStream_t s);
 inline size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Fill the per-warp context for (strip, seg) of the pass described by p.

@@ -243,6 +243,12 @@ void apply_shape_default(ResolvedConfig &rc, int H, int W) {
         rc.T = px < 200000 ? 4 : px < 600000 ? 5 : 4;
 }
 
+// A depth, a segment size or a layout in hs_config asks for the streaming passes; otherwise an
+// image that fits the chip runs in the resident form (hs_resident.cuh).
+static bool wants_resident(const ResolvedConfig &rc) {
+    return rc.T_default && rc.seg_rows == 0 && rc.layout == 0;
+}
+
 // Runs `iters` sweeps.  State starts in (u0, v0) if `start_in_user`, else in (u1, v1);
 // the final state always lands in (u0, v0).
 hs_status run_passes_dev(const float *Ix, const float *Iy, const float *It, int H, int W, int ld,
@@ -322,6 +328,11 @@ hs_status hs_sweeps(const float *Ix, const float *Iy, const float *It, int H, in
     float *u1 = reinterpret_cast<float *>(workspace);
     float *v1 = reinterpret_cast<float *>(reinterpret_cast<char *>(workspace) + pb);
     cudaStream_t s = (cudaStream_t)stream;
+    ResidentPlan pl;
+    if (wants_resident(rc) && resident_plan(H, W, iters, workspace_bytes, pl)) {
+        st = run_resident(nullptr, nullptr, Ix, Iy, It, H, W, ld, alpha2, iters, u, v, workspace, false, rc, pl, s);
+        if (st != HS_ERR_UNSUPPORTED) return st;
+    }
     const int passes = (iters + rc.T - 1) / rc.T;
     if (passes % 2 == 1) {
         // the state must start in the scratch pair so that the last pass ends in (u, v)
@@ -357,6 +368,12 @@ hs_status hs_forward(const float *I0, const float *I1, int H, int W, int ld, flo
     float *u1 = reinterpret_cast<float *>(w + 3 * pb);
     float *v1 = reinterpret_cast<float *>(w + 4 * pb);
     cudaStream_t s = (cudaStream_t)stream;
+    ResidentPlan pl;
+    if (wants_resident(rc) && resident_plan(H, W, iters, need, pl)) {
+        st = run_resident(I0, I1, nullptr, nullptr, nullptr, H, W, ld, alpha * alpha, iters, u, v, workspace, true,
+                          rc, pl, s);
+        if (st != HS_ERR_UNSUPPORTED) return st;
+    }
     if ((st = hs_derivs(I0, I1, H, W, ld, Ix, Iy, It, stream)) != HS_OK) return st;
     const int passes = iters > 0 ? (iters + rc.T - 1) / rc.T : 0;
     // zero the buffer pair the first pass reads (u, v themselves when no pass runs)

@@ -55,10 +55,13 @@ typedef enum hs_binop { HS_OP_ADD = 0, HS_OP_SUB = 1, HS_OP_MUL = 2, HS_OP_DIV =
 /* Tuning of the sweep kernels.  Zero-initialise for the defaults. */
 typedef struct hs_config {
     int sweeps_per_pass;  /* temporal-blocking depth T (1..8) = sweeps per HBM pass; 0 = default:
-                           * for hs_forward / hs_sweeps / hs_forward_noalloc a measured table by
-                           * image size and form (within 6 % of the autotuned best on B200 from
-                           * 240x320 to 4096^2, 16 % at 512^2 in the fast form), 4 for the
-                           * other calls */
+                           * for hs_forward / hs_sweeps / hs_forward_noalloc, when
+                           * rows_per_segment and layout are 0 too, an image that the SMs can hold
+                           * at once (about 2 Mpx) stays on the chip for all sweeps, one tile per
+                           * SM in a cooperative launch (results are the same bit for bit);
+                           * otherwise a measured table by image size and form (within 6 % of the
+                           * autotuned best on B200 from 240x320 to 4096^2, 16 % at 512^2 in the
+                           * fast form), 4 for the other calls */
     int rows_per_segment; /* rows each warp streams per work item; 0 = default */
     int fast_math;        /* 0 (default): the reference program's operation order, one
                              rounding per operation -- bit-identical to the reference's

@@ -12,6 +12,7 @@
 // registers run it faster than 8 of 255 (1.72 against 2.14 us per sweep): the state of R = 16
 // rows leaves too few warps to cover the shuffles.
 #include <algorithm>
+#include <cstring>
 #include <mutex>
 
 #include "hs_resident.cuh"
@@ -41,23 +42,6 @@ __device__ __forceinline__ void msg_load(const float4 *p, float (&f)[3], unsigne
         : "memory");
 }
 
-// The lane's 4 columns of a row, the first n of them when the image ends inside the chunk
-// (columns past W may belong to other data of the caller).
-__device__ __forceinline__ void res_store(float *U, float *V, size_t off, int n, const float2 (&c)[2][2]) {
-    if (n >= 4) {
-        *reinterpret_cast<float4 *>(U + off) = cat4(c[0][0], c[0][1]);
-        *reinterpret_cast<float4 *>(V + off) = cat4(c[1][0], c[1][1]);
-    } else {
-        const float a[3] = {c[0][0].x, c[0][0].y, c[0][1].x}, b[3] = {c[1][0].x, c[1][0].y, c[1][1].x};
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-            if (j < n) {
-                U[off + j] = a[j];
-                V[off + j] = b[j];
-            }
-    }
-}
-
 // A chunk (8 floats, 16-byte aligned) to and from the lane's columns of a row.
 __device__ __forceinline__ void put_chunk(float *s, const float2 (&c)[2][2]) {
     reinterpret_cast<float4 *>(s)[0] = cat4(c[0][0], c[0][1]);
@@ -83,7 +67,7 @@ struct ResSmem {
 };
 
 template <bool FAST, int NW, int R>
-__global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_constant__ ResidentParams p) {
+__global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_constant__ ResidentTable tab) {
     using S = ResSmem<NW, R>;
     extern __shared__ float4 smem[];
     __shared__ unsigned tmem_base;
@@ -92,21 +76,18 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
     float *out = reinterpret_cast<float *>(smem) + S::out / 4, *in = reinterpret_cast<float *>(smem) + S::in / 4;
     int *src = reinterpret_cast<int *>(smem) + S::src / 4;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int kWords = (NW / 4) * R * 16;
-    constexpr int kTmemCols = kWords <= 32 ? 32 : kWords <= 64 ? 64 : kWords <= 128 ? 128 : kWords <= 256 ? 256 : 512;
-    static_assert(kWords <= 512, "the coefficients of a tile fit tensor memory");
+    constexpr int kCols = res_tmem_cols<NW, R>();
     if (warp == 0) {
-        const unsigned s = (unsigned)__cvta_generic_to_shared(&tmem_base);
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s), "n"(kTmemCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+        tmem_alloc(&tmem_base, kCols);
         if (lane == 0) stop = 0;
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const unsigned tmem = tmem_base_of(&tmem_base);
 
-    const int tile = blockIdx.x, tx = tile % p.ntx, ty = tile / p.ntx;
+    int image = 0;
+    while (image + 1 < tab.n && tab.first[image + 1] <= (int)blockIdx.x) ++image;
+    const ResImage &p = tab.img[image];
+    const int tile = blockIdx.x - tab.first[image], tx = tile % p.ntx, ty = tile / p.ntx;
+    const float alpha2 = p.alpha_dev ? __fmul_rn(__ldg(p.alpha_dev), __ldg(p.alpha_dev)) : p.alpha2;
     const int chunks = (p.W + 3) / 4;
     const int x0 = 4 * res_split(tx, p.ntx, chunks), x1 = 4 * res_split(tx + 1, p.ntx, chunks);
     const int y0 = res_split(ty, p.nty, p.H), y1 = res_split(ty + 1, p.nty, p.H);
@@ -120,7 +101,7 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
     t.last = xa <= p.W - 1 && xa + 4 > p.W - 1;
     t.row0 = y0 - kResT + warp * R;
     t.H = p.H;
-    t.tmem = tmem_base + ((unsigned)(warp & 3) << 21) + (unsigned)(warp >> 2) * (R * 16);
+    t.tmem = tmem + ((unsigned)(warp & 3) << 21) + (unsigned)(warp >> 2) * (R * 16);
     // every plane row holds whole chunks (ld % 4 == 0), so a chunk that starts inside the image
     // may be read; other chunks are never needed
     const bool col_in = xa >= 0 && xa < p.W;
@@ -160,6 +141,11 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
                 const float b[4] = {i1[j], i1[j + 1], n1[j], n1[j + 1]};
                 hs_derivs_taps(a, b, c[j], c[4 + j], c[8 + j]);
             }
+            if (p.Ix && own_col && row >= y0 && row < y1) {  // (scratch planes: whole chunks)
+                *reinterpret_cast<float4 *>(p.Ix + off) = make_float4(c[0], c[1], c[2], c[3]);
+                *reinterpret_cast<float4 *>(p.Iy + off) = make_float4(c[4], c[5], c[6], c[7]);
+                *reinterpret_cast<float4 *>(p.It + off) = make_float4(c[8], c[9], c[10], c[11]);
+            }
 #pragma unroll
             for (int j = 0; j < 5; ++j) {
                 i0[j] = n0[j];
@@ -173,25 +159,9 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
             c[4] = iy.x; c[5] = iy.y; c[6] = iy.z; c[7] = iy.w;
             c[8] = it.x; c[9] = it.y; c[10] = it.z; c[11] = it.w;
         }
-        // cells outside the image: never used, but the exact form's division should see ordinary
-        // numbers (a zero numerator takes the division's slow branch for the whole warp)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (!in) {
-                c[j] = c[4 + j] = 0.f;
-                c[8 + j] = 1.f;
-            }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if constexpr (FAST) {
-                c[12 + j] = -rcp_approx(fmaf(c[4 + j], c[4 + j], fmaf(c[j], c[j], p.alpha2)));
-            } else {
-                c[12 + j] = -__fadd_rn(__fadd_rn(p.alpha2, __fmul_rn(c[j], c[j])), __fmul_rn(c[4 + j], c[4 + j]));
-            }
-        }
-        tmem_st16(t.tmem + 16 * r, c);
+        res_coefficients<FAST>(t.tmem + 16 * r, c, alpha2, in);
         float4 u = z4, v = z4;
-        if (in && !p.zero_start) {
+        if (in && !tab.zero_start) {
             u = __ldcg(reinterpret_cast<const float4 *>(p.u + off));
             v = __ldcg(reinterpret_cast<const float4 *>(p.v + off));
         }
@@ -211,7 +181,7 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
     const bool ghosts = (t.row0 < 0 && t.row0 + R > 0) || (t.row0 < p.H && t.row0 + R > p.H);
     // where each message received comes from: its index in all outboxes' first half, -1: none
     const int half_msgs = p.ntx * p.nty * S::msgs;
-    if (p.nblocks > 1) {
+    if (tab.nblocks > 1) {
         const int lown = nl ? res_split(tx, p.ntx, chunks) - res_split(tx - 1, p.ntx, chunks) : 0;
         for (int i = threadIdx.x; i < S::msgs; i += NW * 32) {
             const int c = i / 3, m = i % 3;
@@ -237,20 +207,37 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
     const int row_end = t.row0 + R;
     const bool up_rows = t.row0 < y0 + kResT && row_end > y0, down_rows = t.row0 < y1 && row_end > y1 - kResT;
     const bool above_rows = t.row0 < y0, below_rows = t.row0 < y1 + kResT && row_end > y1;
-    int done = 0;
-    for (int b = 0; b < p.nblocks; ++b) {
-        const int upto = res_split(b + 1, p.nblocks, p.iters);
-        const int n = upto - done;
-        // (uniform in the CTA; every variant runs one block barrier per sweep)
-        switch (side) {
-            case -1: res_sweeps<FAST, NW, R, -1>(t, cu, pub, done & 1, n, ghosts, p.we, p.wc); break;
-            case 0: res_sweeps<FAST, NW, R, 0>(t, cu, pub, done & 1, n, ghosts, p.we, p.wc); break;
-            case 1: res_sweeps<FAST, NW, R, 1>(t, cu, pub, done & 1, n, ghosts, p.we, p.wc); break;
-            case 2: res_sweeps<FAST, NW, R, 2>(t, cu, pub, done & 1, n, ghosts, p.we, p.wc); break;
-            default: res_sweeps<FAST, NW, R, 3>(t, cu, pub, done & 1, n, ghosts, p.we, p.wc); break;
+    // the tile's own pixels of the state to planes U, V
+    auto store_own = [&](float *U, float *V) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int row = t.row0 + r;
+            if (row >= y0 && row < y1 && own_col) res_store(U, V, (size_t)row * p.ld + xa, p.W - xa, cu[r]);
         }
-        done = upto;
-        if (b + 1 == p.nblocks) break;
+        __syncwarp();
+    };
+    if (p.ckpt) store_own(p.ckpt, p.ckpt + tab.ckpt_plane);  // checkpoint 0: the start state
+    int done = 0, ck = 1;  // ck: the next checkpoint
+    for (int b = 0; b < tab.nblocks; ++b) {
+        const int upto = res_split(b + 1, tab.nblocks, tab.iters);
+        while (done < upto) {
+            const int next = p.ckpt ? min(upto, ck * tab.ckpt_every) : upto, n = next - done;
+            // (uniform in the CTA; every variant runs one block barrier per sweep)
+            switch (side) {
+                case -1: res_sweeps<FAST, NW, R, -1>(t, cu, pub, done & 1, n, ghosts, tab.we, tab.wc); break;
+                case 0: res_sweeps<FAST, NW, R, 0>(t, cu, pub, done & 1, n, ghosts, tab.we, tab.wc); break;
+                case 1: res_sweeps<FAST, NW, R, 1>(t, cu, pub, done & 1, n, ghosts, tab.we, tab.wc); break;
+                case 2: res_sweeps<FAST, NW, R, 2>(t, cu, pub, done & 1, n, ghosts, tab.we, tab.wc); break;
+                default: res_sweeps<FAST, NW, R, 3>(t, cu, pub, done & 1, n, ghosts, tab.we, tab.wc); break;
+            }
+            done = next;
+            if (p.ckpt && (done == ck * tab.ckpt_every || done == tab.iters)) {
+                store_own(p.ckpt + (size_t)(2 * ck) * tab.ckpt_plane, p.ckpt + (size_t)(2 * ck + 1) * tab.ckpt_plane);
+                ++ck;
+            }
+        }
+        if (b + 1 == tab.nblocks) break;
+        if (p.ntx * p.nty == 1) continue;  // no neighbours
 
         // exchange e: the ring into shared memory
         const unsigned e = (unsigned)(b + 1);
@@ -296,8 +283,8 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
             for (int i = 0; i < kPer; ++i) all = all && tag[i] == e;
             if (all) break;
             if (++polls > kResPolls ||
-                ((polls & 1023) == 0 && (*(volatile int *)&stop || *(volatile unsigned *)p.abort_flag))) {
-                atomicExch(p.abort_flag, 1u);
+                ((polls & 1023) == 0 && (*(volatile int *)&stop || *(volatile unsigned *)tab.abort_flag))) {
+                atomicExch(tab.abort_flag, 1u);
                 *(volatile int *)&stop = 1;
                 break;
             }
@@ -334,7 +321,7 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
     }
     __syncthreads();
     bool ok = true;
-    if (p.nblocks > 1) ok = stop == 0 && *(volatile unsigned *)p.abort_flag == 0u;
+    if (tab.nblocks > 1) ok = stop == 0 && *(volatile unsigned *)tab.abort_flag == 0u;
     if (!ok) {
         const float2 nan2 = f2(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
 #pragma unroll
@@ -342,20 +329,15 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
 #pragma unroll
             for (int q = 0; q < 2; ++q) cu[r][q][0] = cu[r][q][1] = nan2;
     }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int row = t.row0 + r;
-        if (row >= y0 && row < y1 && own_col) res_store(p.u, p.v, (size_t)row * p.ld + xa, p.W - xa, cu[r]);
-    }
+    store_own(p.u, p.v);
     __syncthreads();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(kTmemCols));
+    if (warp == 0) tmem_dealloc(tmem, kCols);
 }
 
 // ------------------------------------------------------------------ host side
 
 template <bool FAST, int NW, int R>
-static hs_status launch_resident(const ResidentParams &p, cudaStream_t s) {
+static hs_status launch_resident(const ResidentTable &tab, cudaStream_t s) {
     auto fn = hs_resident_kernel<FAST, NW, R>;
     constexpr int smem = ResSmem<NW, R>::bytes;
     static std::mutex mu;
@@ -370,7 +352,7 @@ static hs_status launch_resident(const ResidentParams &p, cudaStream_t s) {
         }
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(p.ntx * p.nty));
+    cfg.gridDim = dim3((unsigned)tab.first[tab.n]);
     cfg.blockDim = dim3(NW * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
@@ -379,7 +361,7 @@ static hs_status launch_resident(const ResidentParams &p, cudaStream_t s) {
     a[0].val.cooperative = 1;
     cfg.attrs = a;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, p);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, tab);
     if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs at hand than the device has
         cudaGetLastError();
         return HS_ERR_UNSUPPORTED;
@@ -388,65 +370,167 @@ static hs_status launch_resident(const ResidentParams &p, cudaStream_t s) {
     return HS_OK;
 }
 
-struct ResShape {
-    int nw, r;
-    int rows() const { return nw * r - 2 * kResT; }  // a tile's own rows, at most
-};
-constexpr ResShape kResShapes[] = {{16, 2}, {16, 3}, {16, 4}, {16, 5}, {16, 6}, {16, 7}, {16, 8}};
+// Tile shapes: 16 warps of r rows; a tile's own rows, at most.
+constexpr int kResWarps = 16, kResMinR = 2, kResMaxR = 8;
+constexpr int res_rows(int r) { return kResWarps * r - 2 * kResT; }
 
-// Scratch of a tiling: both halves of every tile's outbox, then the abort flag.
-static size_t box_bytes(const ResidentPlan &pl) {
-    if (pl.ntx * pl.nty == 1) return 0;
-    return (size_t)2 * pl.ntx * pl.nty * res_msgs(pl.nw * pl.r) * sizeof(float4) + 256;
+int resident_tiles(int H, int W, int r, int *ntx, int *nty) {
+    const int chunks = (W + 3) / 4;
+    *ntx = (chunks + kResChunks - 1) / kResChunks;
+    *nty = (H + res_rows(r) - 1) / res_rows(r);
+    const long tiles = (long)*ntx * *nty;
+    return (int)std::min(tiles, 1L << 30);
+}
+
+size_t resident_box_bytes(int tiles, int r) {
+    if (tiles == 1) return 0;
+    return (size_t)2 * tiles * res_msgs(kResWarps * r) * sizeof(float4) + 256;
 }
 
 // The tiling of an H x W image: the smallest tiles that the SMs hold all at once and whose
 // outboxes fit the scratch.
 bool resident_plan(int H, int W, int iters, size_t scratch_bytes, ResidentPlan &pl) {
     if (iters < 2) return false;
-    const int chunks = (W + 3) / 4;
-    pl.ntx = (chunks + kResChunks - 1) / kResChunks;
-    const int sms = sm_count();
-    for (const ResShape &s : kResShapes) {
-        pl.nw = s.nw;
-        pl.r = s.r;
-        pl.nty = (H + s.rows() - 1) / s.rows();
-        if ((long)pl.ntx * pl.nty > sms) continue;
-        pl.box_bytes = box_bytes(pl);
-        if (pl.box_bytes > scratch_bytes) continue;
-        // several tiles: at least one exchange, so that no tile writes its result before its
-        // neighbours have read their inputs; a single tile needs none
-        pl.nblocks = pl.ntx * pl.nty == 1 ? 1 : std::max(2, (iters + kResT - 1) / kResT);
-        return true;
+    for (int r = kResMinR; r <= kResMaxR; ++r) {
+        const int tiles = resident_tiles(H, W, r, &pl.ntx, &pl.nty);
+        if (tiles > sm_count()) continue;
+        pl.r = r;
+        pl.box_bytes = resident_box_bytes(tiles, r);
+        if (pl.box_bytes <= scratch_bytes) return true;
     }
     return false;
+}
+
+// Launches the table (img, n, ckpt_* filled in; the tiling per image for r rows per warp).
+// Several tiles: at least one exchange, so that no tile writes its result before its neighbours
+// have read their inputs; images of a single tile need none.
+static hs_status launch_table(ResidentTable &tab, int r, int iters, bool zero_start, const ResolvedConfig &rc,
+                              cudaStream_t s) {
+    tab.first[0] = 0;
+    bool several = false;
+    for (int i = 0; i < tab.n; ++i) {
+        const int tiles = tab.img[i].ntx * tab.img[i].nty;
+        tab.first[i + 1] = tab.first[i] + tiles;
+        several |= tiles > 1;
+    }
+    tab.we = rc.we;
+    tab.wc = rc.wc;
+    tab.iters = iters;
+    tab.nblocks = several ? std::max(2, (iters + kResT - 1) / kResT) : 1;
+    tab.zero_start = zero_start ? 1 : 0;
+    switch (r) {
+#define HS_RES(RR) \
+    case RR: return rc.fast ? launch_resident<true, kResWarps, RR>(tab, s) : launch_resident<false, kResWarps, RR>(tab, s);
+        HS_RES(2) HS_RES(3) HS_RES(4) HS_RES(5) HS_RES(6) HS_RES(7) HS_RES(8)
+#undef HS_RES
+    }
+    HS_FAIL(HS_ERR_INVALID_ARG, "internal: no resident kernel for %d rows", r);
 }
 
 hs_status run_resident(const float *I0, const float *I1, const float *Ix, const float *Iy, const float *It, int H,
                        int W, int ld, float alpha2, int iters, float *u, float *v, void *scratch, bool zero_start,
                        const ResolvedConfig &rc, const ResidentPlan &pl, cudaStream_t s) {
-    ResidentParams p;
+    ResidentTable tab;
+    memset(&tab, 0, sizeof(tab));
+    tab.n = 1;
+    ResImage &p = tab.img[0];
     p.I0 = I0; p.I1 = I1;
-    p.Ix = Ix; p.Iy = Iy; p.It = It;
+    p.Ix = const_cast<float *>(Ix); p.Iy = const_cast<float *>(Iy); p.It = const_cast<float *>(It);
     p.u = u; p.v = v;
     p.box = reinterpret_cast<float4 *>(scratch);
-    p.abort_flag = nullptr;
     p.H = H; p.W = W; p.ld = ld;
     p.alpha2 = alpha2;
-    p.we = rc.we; p.wc = rc.wc;
     p.ntx = pl.ntx; p.nty = pl.nty;
-    p.iters = iters; p.nblocks = pl.nblocks;
-    p.zero_start = zero_start ? 1 : 0;
     if (pl.box_bytes) {
         HS_CUDA_CHECK(cudaMemsetAsync(scratch, 0, pl.box_bytes, s));
-        p.abort_flag = reinterpret_cast<unsigned *>(reinterpret_cast<char *>(scratch) + pl.box_bytes - 256);
+        tab.abort_flag = reinterpret_cast<unsigned *>(reinterpret_cast<char *>(scratch) + pl.box_bytes - 256);
     }
-#define HS_RES(NWW, RR)                                                                   \
-    if (pl.nw == NWW && pl.r == RR)                                                       \
-        return rc.fast ? launch_resident<true, NWW, RR>(p, s) : launch_resident<false, NWW, RR>(p, s);
-    HS_RES(16, 2) HS_RES(16, 3) HS_RES(16, 4) HS_RES(16, 5) HS_RES(16, 6) HS_RES(16, 7) HS_RES(16, 8)
-#undef HS_RES
-    HS_FAIL(HS_ERR_INVALID_ARG, "internal: no resident kernel for %d x %d", pl.nw, pl.r);
+    return launch_table(tab, pl.r, iters, zero_start, rc, s);
+}
+
+// ---- many images: groups whose tiles the SMs hold all at once, one launch each
+
+// Greedy groups in order with r rows per warp; returns their number, 0 if an image does not fit.
+static int resident_groups(const ResidentJob *jobs, int n, int r, int *group_end) {
+    int groups = 0, tiles = 0;
+    for (int i = 0; i < n; ++i) {
+        int ntx, nty;
+        const int t = resident_tiles(jobs[i].H, jobs[i].W, r, &ntx, &nty);
+        if (t > sm_count() || resident_box_bytes(t, r) > jobs[i].scratch_bytes) return 0;
+        if (tiles + t > sm_count()) {
+            group_end[groups++] = i;
+            tiles = 0;
+        }
+        tiles += t;
+    }
+    group_end[groups++] = n;
+    return groups;
+}
+
+// A sweep of one launch takes about 0.9 + 0.2 r us in the fast form (1080p, 1.9 x the slope in the
+// exact form), whatever the number of tiles; the tile height that needs the least in all.
+int resident_choose(const ResidentJob *jobs, int n, bool fast, int *group_end) {
+    int best_r = 0;
+    double best = 0.0;
+    int ends[kMaxResImages];
+    for (int r = kResMinR; r <= kResMaxR; ++r) {
+        const int g = resident_groups(jobs, n, r, ends);
+        if (g == 0) continue;
+        const double cost = g * (0.9 + (fast ? 0.2 : 0.38) * r);
+        if (best_r == 0 || cost < best) {
+            best_r = r;
+            best = cost;
+        }
+    }
+    if (best_r) resident_groups(jobs, n, best_r, group_end);
+    return best_r;
+}
+
+hs_status run_resident_jobs(const ResidentJob *jobs, int n, int iters, int ckpt_every, size_t ckpt_plane,
+                            const ResolvedConfig &rc, cudaStream_t s) {
+    int ends[kMaxResImages];
+    if (n > kMaxResImages || iters < 2) return HS_ERR_UNSUPPORTED;
+    if (resident_choose(jobs, n, rc.fast, ends) == 0) return HS_ERR_UNSUPPORTED;
+    for (int i0 = 0, g = 0; i0 < n; i0 = ends[g++]) {
+        const int m = ends[g] - i0;
+        int sub[kMaxResImages];
+        // (a last, smaller group may take smaller tiles)
+        int r = 0;
+        for (int q = kResMinR; q <= kResMaxR && !r; ++q)
+            if (resident_groups(jobs + i0, m, q, sub) == 1) r = q;
+        ResidentTable tab;
+        memset(&tab, 0, sizeof(tab));
+        tab.n = m;
+        tab.ckpt_every = ckpt_every;
+        tab.ckpt_plane = ckpt_plane;
+        size_t box = 0;
+        for (int i = 0; i < m; ++i) {
+            const ResidentJob &d = jobs[i0 + i];
+            ResImage &p = tab.img[i];
+            p.I0 = d.I0; p.I1 = d.I1;
+            p.Ix = d.Ix; p.Iy = d.Iy; p.It = d.It;
+            p.u = d.u; p.v = d.v;
+            p.ckpt = d.ckpt;
+            p.box = reinterpret_cast<float4 *>(d.scratch);
+            p.alpha_dev = d.alpha_dev;
+            p.H = d.H; p.W = d.W; p.ld = d.ld;
+            const int tiles = resident_tiles(d.H, d.W, r, &p.ntx, &p.nty);
+            const size_t bytes = resident_box_bytes(tiles, r);
+            if (bytes > box) {
+                box = bytes;
+                tab.abort_flag = reinterpret_cast<unsigned *>(d.scratch + bytes - 256);
+            }
+        }
+        // clear the outboxes: the jobs' scratch buffers lie one stride apart
+        if (box && m == 1) HS_CUDA_CHECK(cudaMemsetAsync(jobs[i0].scratch, 0, box, s));
+        if (box && m > 1) {
+            const size_t pitch = jobs[i0 + 1].scratch - jobs[i0].scratch;
+            HS_CUDA_CHECK(cudaMemset2DAsync(jobs[i0].scratch, pitch, 0, box, m, s));
+        }
+        const hs_status st = launch_table(tab, r, iters, true, rc, s);
+        if (st != HS_OK) return st;
+    }
+    return HS_OK;
 }
 
 }  // namespace hs

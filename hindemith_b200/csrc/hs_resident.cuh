@@ -46,16 +46,29 @@ constexpr int kResT = 4;                      // sweeps between exchanges = halo
 constexpr int kResCols = 128;                 // columns of a tile, halo included (4 per lane)
 constexpr int kResChunks = kResCols / 4 - 2;  // 4-column chunks of a tile's own region, at most
 
-struct ResidentParams {
+constexpr int kMaxResImages = 32;  // images of one launch
+
+struct ResImage {
     const float *I0, *I1;        // if set: the images; the kernel forms the derivatives itself
-    const float *Ix, *Iy, *It;   // else the derivative planes
+    float *Ix, *Iy, *It;         // else the derivative planes; with the images: where to keep them, or null
     float *u, *v;                // state: read at the start (unless zero_start), written at the end
-    float4 *box;                 // outboxes of all tiles, then one word: the abort flag
-    unsigned *abort_flag;
-    int H, W, ld;
+    float *ckpt;                 // if set: checkpoint c, the state after c * ckpt_every sweeps and at
+                                 // the end, goes to plane 2c (u) and 2c + 1 (v) from here
+    float4 *box;                 // outboxes of the image's tiles
+    const float *alpha_dev;      // if set, alpha2 = alpha_dev[0] squared
     float alpha2;
-    float we, wc;
+    int H, W, ld;
     int ntx, nty;                // tiles across and down
+};
+
+struct ResidentTable {
+    ResImage img[kMaxResImages];
+    int first[kMaxResImages + 1];  // tiles of the images before image i
+    int n;
+    unsigned *abort_flag;
+    size_t ckpt_plane;           // floats between checkpoint planes
+    int ckpt_every;
+    float we, wc;
     int iters, nblocks;          // the sweeps run in nblocks blocks of at most kResT
     int zero_start;
 };
@@ -83,8 +96,7 @@ __device__ __forceinline__ void tmem_st16(unsigned addr, const float (&r)[16]) {
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
         "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"f"(r[0]), "f"(r[1]), "f"(r[2]),
         "f"(r[3]), "f"(r[4]), "f"(r[5]), "f"(r[6]), "f"(r[7]), "f"(r[8]), "f"(r[9]), "f"(r[10]),
-        "f"(r[11]), "f"(r[12]), "f"(r[13]), "f"(r[14]), "f"(r[15]), "r"(addr)
-        : "memory");
+        "f"(r[11]), "f"(r[12]), "f"(r[13]), "f"(r[14]), "f"(r[15]), "r"(addr));
 }
 __device__ __forceinline__ void tmem_ld16(float (&r)[16], unsigned addr) {
     asm volatile(
@@ -336,6 +348,72 @@ __device__ __forceinline__ void res_sweeps(const ResLane &t, float2 (&cu)[R][2][
         if (ghosts) res_ghost_rows<R>(t, cu);
         res_sweep<FAST, NW, R, SIDE>(t, cu, pub + half * (NW * 128), wef, wcf);
     }
+}
+
+// The lane's 4 columns of a row, the first n of them when the image ends inside the chunk
+// (columns past W may belong to other data of the caller).
+__device__ __forceinline__ void res_store(float *U, float *V, size_t off, int n, const float2 (&c)[2][2]) {
+    if (n >= 4) {
+        *reinterpret_cast<float4 *>(U + off) = cat4(c[0][0], c[0][1]);
+        *reinterpret_cast<float4 *>(V + off) = cat4(c[1][0], c[1][1]);
+    } else {
+        const float a[3] = {c[0][0].x, c[0][0].y, c[0][1].x}, b[3] = {c[1][0].x, c[1][0].y, c[1][1].x};
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            if (j < n) {
+                U[off + j] = a[j];
+                V[off + j] = b[j];
+            }
+    }
+}
+
+// A row's coefficients into tensor memory: c holds Ix, Iy, It of the lane's 4 columns, the
+// negated denominator term joins them.
+template <bool FAST>
+__device__ __forceinline__ void res_coefficients(unsigned tmem, float (&c)[16], float alpha2, bool in) {
+    // cells outside the image: never used, but the exact form's division should see ordinary
+    // numbers (a zero numerator takes the division's slow branch for the whole warp)
+    if (!in) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            c[j] = c[4 + j] = 0.f;
+            c[8 + j] = 1.f;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if constexpr (FAST) {
+            c[12 + j] = -rcp_approx(fmaf(c[4 + j], c[4 + j], fmaf(c[j], c[j], alpha2)));
+        } else {
+            c[12 + j] = -__fadd_rn(__fadd_rn(alpha2, __fmul_rn(c[j], c[j])), __fmul_rn(c[4 + j], c[4 + j]));
+        }
+    }
+    tmem_st16(tmem, c);
+}
+
+// Tensor memory of a CTA: one warp allocates `cols` columns (a power of two from 32) for all.
+__device__ __forceinline__ void tmem_alloc(unsigned *base, int cols) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(base);
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s), "r"(cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+}
+// After the allocating warp: every warp sees the base.
+__device__ __forceinline__ unsigned tmem_base_of(const unsigned *base) {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    return *(volatile const unsigned *)base;
+}
+__device__ __forceinline__ void tmem_dealloc(unsigned base, int cols) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols));
+}
+// columns a CTA of NW warps x R rows allocates
+template <int NW, int R>
+constexpr int res_tmem_cols() {
+    constexpr int words = (NW / 4) * R * 16;
+    static_assert(NW % 4 == 0 && words <= 512, "the coefficients of a tile fit tensor memory");
+    return words <= 32 ? 32 : words <= 64 ? 64 : words <= 128 ? 128 : words <= 256 ? 256 : 512;
 }
 
 }  // namespace hs

@@ -420,9 +420,8 @@ hs_status run_passes_dev(const float *Ix, const float *Iy, const float *It, int 
 
 // The resident form (hs_resident.cu): the tiling of an image that fits the chip.
 struct ResidentPlan {
-    int nw, r;         // warps per CTA and rows per warp
+    int r;             // rows per warp
     int ntx, nty;      // tiles across and down
-    int nblocks;       // blocks of sweeps between exchanges
     size_t box_bytes;  // scratch for the exchanges
 };
 // false when the image does not fit (or the call is too short, or the scratch too small): the
@@ -435,6 +434,22 @@ bool resident_plan(int H, int W, int iters, size_t scratch_bytes, ResidentPlan &
 hs_status run_resident(const float *I0, const float *I1, const float *Ix, const float *Iy, const float *It, int H,
                        int W, int ld, float alpha2, int iters, float *u, float *v, void *scratch, bool zero_start,
                        const ResolvedConfig &rc, const ResidentPlan &pl, cudaStream_t s);
+// The resident form for many images (training): derivatives into Ix, Iy, It, the state after
+// every ckpt_every sweeps into the checkpoint planes (ckpt_plane floats apart; u then v), the
+// final state into u, v as well.  The jobs' scratch buffers have one size and lie one stride
+// apart.  HS_ERR_UNSUPPORTED when an image does not fit (any launches made are to be redone).
+struct ResidentJob {
+    const float *I0, *I1;
+    float *Ix, *Iy, *It, *u, *v, *ckpt;
+    char *scratch;
+    size_t scratch_bytes;
+    const float *alpha_dev;
+    int H, W, ld;
+};
+hs_status run_resident_jobs(const ResidentJob *jobs, int n, int iters, int ckpt_every, size_t ckpt_plane,
+                            const ResolvedConfig &rc, cudaStream_t s);
+// A depth, a segment size or a layout in hs_config asks for the streaming passes.
+inline bool wants_resident(const ResolvedConfig &rc) { return rc.T_default && rc.seg_rows == 0 && rc.layout == 0; }
 inline size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Fill the per-warp context for (strip, seg) of the pass described by p.

@@ -243,12 +243,6 @@ void apply_shape_default(ResolvedConfig &rc, int H, int W) {
         rc.T = px < 200000 ? 4 : px < 600000 ? 5 : 4;
 }
 
-// A depth, a segment size or a layout in hs_config asks for the streaming passes; otherwise an
-// image that fits the chip runs in the resident form (hs_resident.cuh).
-static bool wants_resident(const ResolvedConfig &rc) {
-    return rc.T_default && rc.seg_rows == 0 && rc.layout == 0;
-}
-
 // Runs `iters` sweeps.  State starts in (u0, v0) if `start_in_user`, else in (u1, v1);
 // the final state always lands in (u0, v0).
 hs_status run_passes_dev(const float *Ix, const float *Iy, const float *It, int H, int W, int ld,

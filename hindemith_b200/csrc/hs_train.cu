@@ -701,6 +701,20 @@ static void set_segments(PassTable &tab, int T) {
 static hs_status train_forward(const hs_train_pair *pairs, const PairBufs *bufs, int n, int iters,
                                int ckpt_every, const ResolvedConfig &rc, cudaStream_t s) {
     hs_status st;
+    // Images that fit the chip run there for all sweeps (hs_resident.cuh), in groups of as many
+    // as fit at once: one launch instead of one per pass, and no state traffic but the
+    // checkpoints.  The exchange scratch is the passes' ping-pong buffers.
+    if (wants_resident(rc)) {
+        std::vector<ResidentJob> jobs(n);
+        for (int i = 0; i < n; ++i) {
+            const hs_train_pair &d = pairs[i];
+            const PairBufs &B = bufs[i];
+            jobs[i] = {d.I0, d.I1, B.deriv(0), B.deriv(1), B.deriv(2), d.u, d.v, B.ck(0, 0), B.scratch,
+                       4 * B.pb, d.alpha, d.H, d.W, d.ld};
+        }
+        st = run_resident_jobs(jobs.data(), n, iters, ckpt_every, bufs[0].pb / sizeof(float), rc, s);
+        if (st != HS_ERR_UNSUPPORTED) return st;
+    }
     for (int i = 0; i < n; ++i) {
         const hs_train_pair &d = pairs[i];
         const PairBufs &B = bufs[i];

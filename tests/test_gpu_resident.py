@@ -127,3 +127,30 @@ def test_resident_streams_and_graph(cuda):
         torch.cuda.synchronize()
         same(out[0], refs[1][0], "u")
         same(out[1], refs[1][1], "v")
+
+
+@pytest.mark.parametrize("fast", [True, False])
+@pytest.mark.parametrize("shapes,iters,ckpt", [([(24, 31), (70, 130), (300, 401), (1, 9)], 23, 7),
+                                               ([(300, 500)] * 7, 12, 5), ([(250, 130)], 9, 4),
+                                               ([(40, 50), (130, 40)], 2, 1)])
+def test_resident_training_equals_streaming(cuda, shapes, iters, ckpt, fast):
+    """The training forward on the chip (one launch for many images, several groups of them)
+    keeps the same checkpoints: flows and gradients equal those of the streaming passes."""
+    from hindemith_b200.autograd import horn_schunck, horn_schunck_batch
+
+    ims = [planes(s, 2, seed=50 + i) for i, s in enumerate(shapes)]
+    lam = [planes(s, 2, seed=90 + i) for i, s in enumerate(shapes)]
+
+    def run(cfg):
+        a = torch.tensor(0.8, device="cuda", requires_grad=True)
+        xs = [tuple(t.clone().requires_grad_(True) for t in p) for p in ims]
+        outs = ([horn_schunck(*xs[0], a, iters, ckpt, cfg)] if len(xs) == 1 else
+                horn_schunck_batch(xs, a, iters, ckpt, cfg))
+        loss = sum((u * p).sum() + (v * q).sum() for (u, v), (p, q) in zip(outs, lam))
+        return [t for o in outs for t in o], torch.autograd.grad(loss, [t for x in xs for t in x] + [a])
+
+    (f0, g0), (f1, g1) = run(L.make_config(fast_math=fast)), run(L.make_config(fast_math=fast, sweeps_per_pass=4))
+    for a, b in zip(f0, f1):
+        same(a.detach(), b.detach(), "flow")
+    for a, b in zip(g0, g1):
+        assert (a - b).norm() <= 1e-5 * b.norm(), "gradient"

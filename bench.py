@@ -1092,10 +1092,9 @@ def main():
     peak, peak_kind = load_peaks()
     launch_s = t_sweeps / (args.steps * passes)
     achieved = BYTES_PER_PX_PASS * H * W / launch_s / 1e9
-    # the wide kernel's main loop is unrolled from 3 Mpx up (kUnrollPixels in hs_sweep.cu),
-    # the 2-column kernel's at depths 1 and 2
-    big = H * W >= 3000000
-    kernel = (f"hs_stream_w_kernel<{T},{'true' if big else 'false'}>" if wide else
+    # the wide layout's ring is in tensor memory from 3.3 Mpx up (kTmPixels in hs_sweep.cu); the
+    # 2-column kernel's main loop is unrolled at depths 1 and 2
+    kernel = (f"hs_stream_{'tm' if H * W >= 3300000 else 'w'}_kernel<{T}>" if wide else
               f"hs_stream_kernel<{T},{'false' if args.exact else 'true'},"
               f"{'true' if T <= 2 else 'false'}>") if T else "hs_resident_kernel"
     # ncu figures of this very kernel at this shape (profiles/), when one was captured

@@ -23,6 +23,7 @@
 #pragma once
 
 #include "hs_stream.cuh"
+#include "hs_tmem.cuh"
 
 namespace hs {
 
@@ -44,6 +45,7 @@ struct GeoW {
 struct ItemW {
     float *raw;     // [kWideRawSlots][kRawPlanes][128]
     float4 *coef;   // [T+1][4][32]: Ix, Iy, It, -1/den of the lane's 4 columns
+    unsigned tmem;  // the same ring in tensor memory (TM): 16 columns per slot
     int lane;
     int lcol;       // this lane's chunk, clamped to an in-bounds chunk of the row
     int xa;         // first of the lane's 4 columns
@@ -74,7 +76,7 @@ __device__ __forceinline__ float4 lds4(const float *p) { return *reinterpret_cas
 // column W-1 is always a lane's last column (chunks start at multiples of 4), so only the
 // first column's left clamp and the last column's right clamp can apply.
 // DUMP (the training recompute) also writes every stage's sweep to p.dump_u/v.
-template <int T, int XE, bool EDGE, bool HEAD = false, bool DUMP = false>
+template <int T, int XE, bool EDGE, bool HEAD = false, bool DUMP = false, bool TM = false>
 __device__ __forceinline__ void stream_step_w(const SweepParams &p, const ItemW &it,
                                               Win<true> (&w)[T][2][2], int k, int rslot, int cslot,
                                               int kk = 0) {
@@ -94,11 +96,18 @@ __device__ __forceinline__ void stream_step_w(const SweepParams &p, const ItemW 
         nw.y = -rcp_approx(fmaf(iy.y, iy.y, fmaf(ix.y, ix.y, it.alpha2)));
         nw.z = -rcp_approx(fmaf(iy.z, iy.z, fmaf(ix.z, ix.z, it.alpha2)));
         nw.w = -rcp_approx(fmaf(iy.w, iy.w, fmaf(ix.w, ix.w, it.alpha2)));
-        float4 *cs = it.coef + cslot * 128 + it.lane;
-        cs[0] = ix;
-        cs[32] = iy;
-        cs[64] = t4;
-        cs[96] = nw;
+        if constexpr (TM) {
+            const float c[16] = {ix.x, ix.y, ix.z, ix.w, iy.x, iy.y, iy.z, iy.w,
+                                 t4.x, t4.y, t4.z, t4.w, nw.x, nw.y, nw.z, nw.w};
+            tmem_wait_st();  // the previous step's slot, read in this step
+            tmem_st16(it.tmem + 16 * cslot, c);
+        } else {
+            float4 *cs = it.coef + cslot * 128 + it.lane;
+            cs[0] = ix;
+            cs[32] = iy;
+            cs[64] = t4;
+            cs[96] = nw;
+        }
     }
     // [plane][pair]: pair 0 holds columns (0, 1), pair 1 columns (2, 3)
     float2 cu[2][2] = {{make_float2(u4.x, u4.y), make_float2(u4.z, u4.w)},
@@ -109,6 +118,10 @@ __device__ __forceinline__ void stream_step_w(const SweepParams &p, const ItemW 
     for (int s = 0; s < T; ++s) {
         if (HEAD && kk < 2 * s) break;  // warp-uniform; later stages start later still
         const int n = k - s;  // arriving row (input of sweep s+1)
+        int rs = cslot - (s + 1);
+        if (rs < 0) rs += GeoW<T>::coef_slots;
+        float cm[16];
+        if constexpr (TM) tmem_ld16(cm, it.tmem + 16 * rs);
         float2 ub[2][2];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -132,10 +145,20 @@ __device__ __forceinline__ void stream_step_w(const SweepParams &p, const ItemW 
             ub[q][0] = win_step_h<EDGE>(w[s][q][0], hE, E, n, p.H, we2, wc2);
             ub[q][1] = win_step_h<EDGE>(w[s][q][1], hO, O, n, p.H, we2, wc2);
         }
-        int rs = cslot - (s + 1);
-        if (rs < 0) rs += GeoW<T>::coef_slots;
-        const float4 *cr = it.coef + rs * 128 + it.lane;
-        const float4 cX = cr[0], cY = cr[32], cT = cr[64], cN = cr[96];
+        float4 cX, cY, cT, cN;
+        if constexpr (TM) {
+            tmem_wait_ld(cm);
+            cX = make_float4(cm[0], cm[1], cm[2], cm[3]);
+            cY = make_float4(cm[4], cm[5], cm[6], cm[7]);
+            cT = make_float4(cm[8], cm[9], cm[10], cm[11]);
+            cN = make_float4(cm[12], cm[13], cm[14], cm[15]);
+        } else {
+            const float4 *cr = it.coef + rs * 128 + it.lane;
+            cX = cr[0];
+            cY = cr[32];
+            cT = cr[64];
+            cN = cr[96];
+        }
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const float2 cx = j ? make_float2(cX.z, cX.w) : make_float2(cX.x, cX.y);
@@ -189,11 +212,12 @@ __device__ __forceinline__ void stream_step_w(const SweepParams &p, const ItemW 
     }
 }
 
-// UNR: the main loop body holds two steps.  The rolled loop is shorter code; with one-warp
-// CTAs on an L2-resident image, where
-// instruction fetch is the leading stall, it measured faster (1080p T = 6: 511 against 500
-// Gpix-it/s), the unrolled one on images larger than L2 (4096^2 T = 5: 822 against 805).
-template <int T, int XE, bool DUMP, bool UNR = true>
+// UNR: the main loop body holds two steps.  The rolled loop is shorter code; with one-warp CTAs on
+// an L2-resident image, where instruction fetch is the leading stall, it measured faster (1080p
+// T = 6: 511 against 500 Gpix-it/s), the unrolled one on images larger than L2 (4096^2 T = 5: 822
+// against 805).
+// TM: the coefficient ring is in tensor memory (it.tmem), not in shared memory.
+template <int T, int XE, bool DUMP, bool UNR = true, bool TM = false>
 __device__ __forceinline__ void stream_item_w(const SweepParams &p, const ItemW &it) {
     const int k0 = max(0, it.y_start - T);
     const int k_end = it.y_end - 1 + T;
@@ -224,23 +248,23 @@ __device__ __forceinline__ void stream_item_w(const SweepParams &p, const ItemW 
     // 2T-2 steps skip those stages, T(T-1) stage-steps per segment.
     if (!DUMP && k0 >= T && k0 + 2 * T - 2 <= khi) {  // (dump passes: as the 2-column kernel)
         for (int kk = 0; kk < 2 * T - 2; ++kk, advance())
-            stream_step_w<T, XE, false, true>(p, it, w, k, rslot, cslot, kk);
+            stream_step_w<T, XE, false, true, false, TM>(p, it, w, k, rslot, cslot, kk);
     }
     if (klo + 1 <= khi) {
-        for (; k < klo; advance()) stream_step_w<T, XE, true, false, DUMP>(p, it, w, k, rslot, cslot);
+        for (; k < klo; advance()) stream_step_w<T, XE, true, false, DUMP, TM>(p, it, w, k, rslot, cslot);
         if constexpr (UNR) {
             while (k + 1 <= khi) {
-                stream_step_w<T, XE, false, false, DUMP>(p, it, w, k, rslot, cslot);
+                stream_step_w<T, XE, false, false, DUMP, TM>(p, it, w, k, rslot, cslot);
                 advance();
-                stream_step_w<T, XE, false, false, DUMP>(p, it, w, k, rslot, cslot);
+                stream_step_w<T, XE, false, false, DUMP, TM>(p, it, w, k, rslot, cslot);
                 advance();
             }
         } else {
 #pragma unroll 1
-            for (; k <= khi; advance()) stream_step_w<T, XE, false, false, DUMP>(p, it, w, k, rslot, cslot);
+            for (; k <= khi; advance()) stream_step_w<T, XE, false, false, DUMP, TM>(p, it, w, k, rslot, cslot);
         }
     }
-    for (; k <= k_end; advance()) stream_step_w<T, XE, true, false, DUMP>(p, it, w, k, rslot, cslot);
+    for (; k <= k_end; advance()) stream_step_w<T, XE, true, false, DUMP, TM>(p, it, w, k, rslot, cslot);
     cp_async_wait<0>();
 }
 
@@ -271,14 +295,14 @@ __device__ __forceinline__ void init_item_w(ItemW &it, const SweepParams &p, int
     it.alpha2 = p.alpha_dev ? __fmul_rn(__ldg(p.alpha_dev), __ldg(p.alpha_dev)) : p.alpha2;
 }
 
-template <int T, bool DUMP = false, bool UNR = true>
+template <int T, bool DUMP = false, bool UNR = true, bool TM = false>
 __device__ __forceinline__ void run_item_w(const SweepParams &p, const ItemW &it) {
     const int x0 = it.xa - 4 * it.lane;
     if (x0 <= 0 || x0 + kWideCols >= p.W) {
-        if ((p.W & 3) == 0) stream_item_w<T, 2, DUMP, UNR>(p, it);
-        else stream_item_w<T, 1, DUMP, UNR>(p, it);
+        if ((p.W & 3) == 0) stream_item_w<T, 2, DUMP, UNR, TM>(p, it);
+        else stream_item_w<T, 1, DUMP, UNR, TM>(p, it);
     } else {
-        stream_item_w<T, 0, DUMP, UNR>(p, it);
+        stream_item_w<T, 0, DUMP, UNR, TM>(p, it);
     }
 }
 

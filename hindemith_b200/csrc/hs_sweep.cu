@@ -29,10 +29,10 @@ __global__ void __launch_bounds__(kPassWarps * 32, res_warps(T) / kPassWarps)
     run_item<T, FAST, false, UNR>(p, it);
 }
 
-// The fast form in the wide layout (hs_stream4.cuh).
+// The fast form in the wide layout (hs_stream4.cuh), one-warp CTAs.
 constexpr int res_warps_w(int T) { return T <= 4 ? 12 : 8; }
 
-template <int T, bool UNR>
+template <int T>
 __global__ void __launch_bounds__(kPassWarps * 32, res_warps_w(T) / kPassWarps)
     hs_stream_w_kernel(const SweepParams p) {
     extern __shared__ float4 smem4[];
@@ -47,7 +47,40 @@ __global__ void __launch_bounds__(kPassWarps * 32, res_warps_w(T) / kPassWarps)
     if (item >= p.nitems) return;  // warp-uniform
     ItemW it;
     init_item_w<T>(it, p, item % p.nstrips, item / p.nstrips, lane, wbase);
-    run_item_w<T, false, UNR>(p, it);
+    run_item_w<T, false, false>(p, it);
+}
+
+// The same with the coefficient ring in tensor memory instead of shared memory: the ring's four
+// 16-byte loads per stage were more than half of the shared-memory traffic that the shuffles
+// wait behind.  A warp reaches the tensor-memory lanes of its rank in the CTA, so a CTA has four
+// warps, which share one allocation.  The main loop is unrolled two steps.  Measured on B200,
+// T = 6 / 7, Gpix-it/s, ring in shared memory -> tensor memory: 2048^2 583 -> 645 / 592 -> 630,
+// 3840x2160 560 -> 590 / 588 -> 610, 4096^2 770 -> 838 / 839 -> 881.
+constexpr int kTmWarps = 4;
+template <int T>
+constexpr int tm_cols() { return (T + 1) * 16 <= 32 ? 32 : (T + 1) * 16 <= 64 ? 64 : (T + 1) * 16 <= 128 ? 128 : 256; }
+
+template <int T>
+__global__ void __launch_bounds__(kTmWarps * 32, res_warps_w(T) / kTmWarps)
+    hs_stream_tm_kernel(const SweepParams p) {
+    __shared__ float4 raw[kTmWarps * GeoW<T>::raw_floats / 4];
+    __shared__ unsigned tmem_base;
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    if (warp == 0) tmem_alloc(&tmem_base, tm_cols<T>());
+    const unsigned tmem = tmem_base_of(&tmem_base);
+    griddep_launch_dependents();
+    griddep_wait();
+    const int item = blockIdx.x * kTmWarps + warp;
+    if (item < p.nitems) {  // warp-uniform
+        ItemW it;
+        init_item_w<T>(it, p, item % p.nstrips, item / p.nstrips, lane,
+                       reinterpret_cast<float *>(raw) + warp * GeoW<T>::raw_floats);
+        it.tmem = tmem + ((unsigned)warp << 21);
+        run_item_w<T, false, true, true>(p, it);
+    }
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem, tm_cols<T>());
 }
 
 // ------------------------------------------------------------------ host side
@@ -76,19 +109,30 @@ static hs_status launch_kernel(KernelFn fn, int smem, bool *attr_set, const Swee
     return HS_OK;
 }
 
-// Images below this size (L2-resident) run the wide kernel's main loop rolled, larger ones
-// unrolled two steps (stream_item_w); measured on B200 (fast form, T = 7): 1080p 521 against
-// 502 Gpix-it/s rolled, 2048^2 605 against 608, 2560x1440 536 against 546, 4096^2 900 against
-// 918.
-constexpr long kUnrollPixels = 3000000;
+// From this size on the wide layout runs with its ring in tensor memory; smaller images keep
+// one-warp CTAs with a rolled main loop (1080p, T = 7: 521 Gpix-it/s rolled against 502 unrolled;
+// four-warp CTAs 8 % behind one-warp ones; T = 7: 1700x1500 536 one-warp against 492 with the ring
+// in tensor memory, 2043x1543 528 against 511, 1700x2000 601 against 610).
+constexpr long kTmPixels = 3300000;
 
 template <int T>
 static hs_status launch_one_w(const SweepParams &pp, cudaStream_t stream) {
-    static bool attr_set[64] = {}, attr_set_r[64] = {};
-    constexpr int smem = kPassWarps * GeoW<T>::warp_floats * (int)sizeof(float);
-    if ((long)pp.H * pp.W >= kUnrollPixels)
-        return launch_kernel(hs_stream_w_kernel<T, true>, smem, attr_set, pp, stream);
-    return launch_kernel(hs_stream_w_kernel<T, false>, smem, attr_set_r, pp, stream);
+    if ((long)pp.H * pp.W < kTmPixels) {
+        static bool attr_set[64] = {};
+        return launch_kernel(hs_stream_w_kernel<T>, kPassWarps * GeoW<T>::warp_floats * (int)sizeof(float), attr_set,
+                             pp, stream);
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((pp.nitems + kTmWarps - 1) / kTmWarps));
+    cfg.blockDim = dim3(kTmWarps * 32);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    HS_CUDA_CHECK(cudaLaunchKernelEx(&cfg, hs_stream_tm_kernel<T>, pp));
+    return HS_OK;
 }
 
 int strip_cols_wide(int T) {
@@ -171,19 +215,20 @@ hs_status launch_pass(int T, bool fast, const SweepParams &pp, cudaStream_t s) {
     HS_FAIL(HS_ERR_INVALID_ARG, "sweeps_per_pass=%d outside 1..%d", T, HS_MAX_SWEEPS_PER_PASS);
 }
 
-// Rows per work item: enough items for about one full wave of resident warps, but
-// never so few rows that the 2T-row halo dominates.
+// Rows per work item: as many items as the SMs hold at once and not one more (a single item in a
+// second wave costs the pass nearly half as much again: 3840x2160, T = 6, 1190 items for 1184
+// slots 581 Gpix-it/s, 1155 items 791; 2048^2 643 -> 695), but never so few rows that the 2T-row
+// halo dominates.
 static int seg_rows_for(int H, int nstrips, int T, long warps_per_sm) {
     const long target = (long)sm_count() * warps_per_sm;
-    long nseg = (target + nstrips - 1) / nstrips;
-    if (nseg < 1) nseg = 1;
+    const long nseg = std::max(1L, target / nstrips);
     int L = (int)((H + nseg - 1) / nseg);
     L = std::max(L, 2 * T);
     L = std::max(L, 8);
     return std::min(L, H);
 }
 
-int default_seg_rows(int H, int nstrips, int T) { return seg_rows_for(H, nstrips, T, 16); }
+int default_seg_rows(int H, int nstrips, int T) { return seg_rows_for(H, nstrips, T, res_warps(T)); }
 
 // Measured on B200: in a launch of several pairs (the batch and the training passes) the wide
 // layout wins from about a 1080p image up (4096^2: 700 vs 592 Gpix-it/s), the narrow one below
@@ -270,7 +315,7 @@ hs_status run_passes_dev(const float *Ix, const float *Iy, const float *It, int 
         const int sc = wide ? strip_cols_wide(t) : strip_cols_for(t);
         pp.nstrips = (W + sc - 1) / sc;
         pp.seg_rows = rc.seg_rows > 0 ? std::min(rc.seg_rows, H)
-                                      : seg_rows_for(H, pp.nstrips, t, wide ? res_warps_w(t) : 16);
+                                      : seg_rows_for(H, pp.nstrips, t, wide ? res_warps_w(t) : res_warps(t));
         const int nseg = (H + pp.seg_rows - 1) / pp.seg_rows;
         pp.nitems = pp.nstrips * nseg;
         hs_status st = wide ? launch_pass_w(t, pp, stream) : launch_pass(t, rc.fast, pp, stream);

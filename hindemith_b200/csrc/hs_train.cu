@@ -683,13 +683,24 @@ static void set_segments(PassTable &tab, int T) {
             tab.pair[i].nstrips = (tab.pair[i].W + strip_cols_wide(T) - 1) / strip_cols_wide(T);
     long rows = 0;
     for (int i = 0; i < tab.npairs; ++i) rows += (long)tab.pair[i].nstrips * tab.pair[i].H;
-    const long target = (long)sm_count() * (tab.wide ? (T <= 4 ? 12 : 8) : 16);
+    // (the narrow kernel's resident warps: 16 to depth 4, 12 to 6, 8 beyond)
+    const long target = (long)sm_count() * (tab.wide ? (T <= 4 ? 12 : 8) : (T <= 4 ? 16 : T <= 6 ? 12 : 8));
     int L = (int)std::max(1L, (rows + target - 1) / target);
-    L = std::max(L, 2 * T);
+    L = std::max(L, std::max(8, 2 * T));
+    // each image rounds its last segment up: longer segments until the items are one wave
+    for (;; ++L) {
+        long items = 0;
+        bool more = false;
+        for (int i = 0; i < tab.npairs; ++i) {
+            items += (long)tab.pair[i].nstrips * ((tab.pair[i].H + L - 1) / L);
+            more |= L < tab.pair[i].H;
+        }
+        if (items <= target || !more) break;
+    }
     tab.item_prefix[0] = 0;
     for (int i = 0; i < tab.npairs; ++i) {
         SweepParams &p = tab.pair[i];
-        p.seg_rows = std::min(std::max(L, 8), p.H);
+        p.seg_rows = std::min(L, p.H);
         p.nitems = p.nstrips * ((p.H + p.seg_rows - 1) / p.seg_rows);
         tab.item_prefix[i + 1] = tab.item_prefix[i] + p.nitems;
     }

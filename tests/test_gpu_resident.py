@@ -154,3 +154,19 @@ def test_resident_training_equals_streaming(cuda, shapes, iters, ckpt, fast):
         same(a.detach(), b.detach(), "flow")
     for a, b in zip(g0, g1):
         assert (a - b).norm() <= 1e-5 * b.norm(), "gradient"
+
+
+@pytest.mark.parametrize("shape", [(1811, 2048), (1650, 2003), (2600, 1282)])
+@pytest.mark.parametrize("T", range(1, 9))
+def test_wide_passes_with_the_ring_in_tensor_memory(cuda, shape, T):
+    """From 3.3 Mpx up the wide layout keeps its coefficient ring in tensor memory: equal to the
+    2-column layout bit for bit, at W % 4 = 0, 3 and 2, with partial last passes."""
+    H, W = shape
+    assert H * W >= 3300000
+    Ix, Iy, It, a, b = planes(shape, 5, seed=T)
+    got, ref = [a.clone(), b.clone()], [a.clone(), b.clone()]
+    for pair, layout in ((got, 2), (ref, 1)):
+        pair[:] = [D.as_plane(t) for t in pair]
+        D.hs_sweeps(Ix, Iy, It, 0.3, 2 * T + 1, *pair, L.make_config(fast_math=True, sweeps_per_pass=T, layout=layout))
+    same(got[0], ref[0], "u")
+    same(got[1], ref[1], "v")

@@ -26,6 +26,7 @@
 // A pair whose sweep count is not a multiple of T finishes with one more, shorter pass
 // launched per pair after the persistent kernel.
 #include <algorithm>
+#include <cstring>
 #include <mutex>
 #include <numeric>
 #include <vector>
@@ -416,6 +417,49 @@ hs_status hs_forward_batched(const hs_pair_desc *pairs, int n, void *workspace,
     char *ws = reinterpret_cast<char *>(workspace);
     int *status = device_status ? device_status : reinterpret_cast<int *>(ws + 4);
     unsigned *abort_flag = reinterpret_cast<unsigned *>(ws + 8);
+
+    // No depth, tile or layout asked for: the images that fit the chip run there (hs_resident.cuh),
+    // longest first, as many at a time as the SMs hold, and each larger one in its own passes.  The
+    // persistent kernel below serves explicit settings: its chains of dependent passes leave the
+    // chip idle unless many tiles are independent (measured on B200, fast form, Gpix-it/s, at its
+    // default depth 4 -> this way: 16 mixed pairs 500 -> 660, 3 of 2048^2 423 -> 690, 8 of 640x480
+    // 183 -> 420).
+    if (wants_resident(rc)) {
+        if (device_status) HS_CUDA_CHECK(cudaMemsetAsync(device_status, 0, sizeof(int), s));
+        std::vector<int> in;
+        for (int i = 0; i < n; ++i)
+            if (resident_fits(pairs[i].H, pairs[i].W, pairs[i].iters, 5 * round_up(plane_bytes(pairs[i].H, pairs[i].ld), 256)))
+                in.push_back(i);
+        std::sort(in.begin(), in.end(), [&](int a, int b) {
+            return pairs[a].iters != pairs[b].iters ? pairs[a].iters > pairs[b].iters : a < b;
+        });
+        std::vector<ResidentJob> jobs(in.size());
+        for (size_t k = 0; k < in.size(); ++k) {
+            const hs_pair_desc &d = pairs[in[k]];
+            ResidentJob &j = jobs[k];
+            memset(&j, 0, sizeof(j));
+            j.I0 = d.I0; j.I1 = d.I1;
+            j.u = d.u; j.v = d.v;
+            j.scratch = ws + plan[in[k]].off_planes;
+            j.scratch_bytes = 5 * round_up(plane_bytes(d.H, d.ld), 256);
+            j.alpha2 = d.alpha * d.alpha;
+            j.H = d.H; j.W = d.W; j.ld = d.ld;
+            j.iters = d.iters;
+        }
+        st = jobs.empty() ? HS_OK : run_resident_jobs(jobs.data(), (int)jobs.size(), 0, 0, device_status, rc, s);
+        if (st != HS_OK && st != HS_ERR_UNSUPPORTED) return st;
+        std::vector<char> done(n, 0);
+        if (st == HS_OK)
+            for (int i : in) done[i] = 1;
+        for (int i = 0; i < n; ++i) {
+            const hs_pair_desc &d = pairs[i];
+            if (done[i]) continue;
+            if ((st = hs_forward(d.I0, d.I1, d.H, d.W, d.ld, d.alpha, d.iters, d.u, d.v, ws + plan[i].off_planes,
+                                 5 * round_up(plane_bytes(d.H, d.ld), 256), cfg, stream)) != HS_OK)
+                return st;
+        }
+        return HS_OK;
+    }
 
     // header and every pair's tile-progress counters start at zero
     HS_CUDA_CHECK(cudaMemsetAsync(ws, 0, kHeaderBytes, s));

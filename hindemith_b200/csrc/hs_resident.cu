@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
+#include <vector>
 
 #include "hs_resident.cuh"
 
@@ -181,7 +182,7 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
     const bool ghosts = (t.row0 < 0 && t.row0 + R > 0) || (t.row0 < p.H && t.row0 + R > p.H);
     // where each message received comes from: its index in all outboxes' first half, -1: none
     const int half_msgs = p.ntx * p.nty * S::msgs;
-    if (tab.nblocks > 1) {
+    if (p.nblocks > 1) {
         const int lown = nl ? res_split(tx, p.ntx, chunks) - res_split(tx - 1, p.ntx, chunks) : 0;
         for (int i = threadIdx.x; i < S::msgs; i += NW * 32) {
             const int c = i / 3, m = i % 3;
@@ -202,6 +203,9 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
             if (nx < 0 || nx >= p.ntx || ny < 0 || ny >= p.nty) from = -1;
             src[i] = from < 0 ? -1 : (ny * p.ntx + nx) * S::msgs + 3 * from + m;
         }
+        // chunks that nobody sends stay 0: cells that are never used, but garbage there (a NaN)
+        // would send whole warps through the exact form's general division
+        for (int i = threadIdx.x; i < S::chunks * 8; i += NW * 32) in[i] = 0.f;
     }
     // (uniform in the warp) rows of the ring, and rows of the halo, among the warp's
     const int row_end = t.row0 + R;
@@ -218,8 +222,8 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
     };
     if (p.ckpt) store_own(p.ckpt, p.ckpt + tab.ckpt_plane);  // checkpoint 0: the start state
     int done = 0, ck = 1;  // ck: the next checkpoint
-    for (int b = 0; b < tab.nblocks; ++b) {
-        const int upto = res_split(b + 1, tab.nblocks, tab.iters);
+    for (int b = 0; b < p.nblocks; ++b) {
+        const int upto = res_split(b + 1, p.nblocks, p.iters);
         while (done < upto) {
             const int next = p.ckpt ? min(upto, ck * tab.ckpt_every) : upto, n = next - done;
             // (uniform in the CTA; every variant runs one block barrier per sweep)
@@ -231,12 +235,12 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
                 default: res_sweeps<FAST, NW, R, 3>(t, cu, pub, done & 1, n, ghosts, tab.we, tab.wc); break;
             }
             done = next;
-            if (p.ckpt && (done == ck * tab.ckpt_every || done == tab.iters)) {
+            if (p.ckpt && (done == ck * tab.ckpt_every || done == p.iters)) {
                 store_own(p.ckpt + (size_t)(2 * ck) * tab.ckpt_plane, p.ckpt + (size_t)(2 * ck + 1) * tab.ckpt_plane);
                 ++ck;
             }
         }
-        if (b + 1 == tab.nblocks) break;
+        if (b + 1 == p.nblocks) break;
         if (p.ntx * p.nty == 1) continue;  // no neighbours
 
         // exchange e: the ring into shared memory
@@ -285,6 +289,7 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
             if (++polls > kResPolls ||
                 ((polls & 1023) == 0 && (*(volatile int *)&stop || *(volatile unsigned *)tab.abort_flag))) {
                 atomicExch(tab.abort_flag, 1u);
+                if (tab.status) atomicCAS(tab.status, 0, (int)HS_ERR_TIMEOUT);
                 *(volatile int *)&stop = 1;
                 break;
             }
@@ -321,7 +326,7 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
     }
     __syncthreads();
     bool ok = true;
-    if (tab.nblocks > 1) ok = stop == 0 && *(volatile unsigned *)tab.abort_flag == 0u;
+    if (p.nblocks > 1) ok = stop == 0 && *(volatile unsigned *)tab.abort_flag == 0u;
     if (!ok) {
         const float2 nan2 = f2(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
 #pragma unroll
@@ -401,23 +406,42 @@ bool resident_plan(int H, int W, int iters, size_t scratch_bytes, ResidentPlan &
     return false;
 }
 
-// Launches the table (img, n, ckpt_* filled in; the tiling per image for r rows per warp).
-// Several tiles: at least one exchange, so that no tile writes its result before its neighbours
-// have read their inputs; images of a single tile need none.
-static hs_status launch_table(ResidentTable &tab, int r, int iters, bool zero_start, const ResolvedConfig &rc,
-                              cudaStream_t s) {
+// Clears the outboxes of a launch's tiles: block i those of tile i.
+__global__ void __launch_bounds__(256) res_clear_kernel(const __grid_constant__ ResidentTable tab, int msgs) {
+    int image = 0;
+    while (image + 1 < tab.n && tab.first[image + 1] <= (int)blockIdx.x) ++image;
+    const ResImage &p = tab.img[image];
+    const int tiles = p.ntx * p.nty, tile = blockIdx.x - tab.first[image];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *tab.abort_flag = 0u;
+    if (tiles == 1) return;
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int h = 0; h < 2; ++h)
+        for (int i = threadIdx.x; i < msgs; i += blockDim.x) p.box[(size_t)(h * tiles + tile) * msgs + i] = z;
+}
+
+// Launches the table (img, n, ckpt_* and abort_flag filled in; every image tiled for r rows per
+// warp).  An image of several tiles has at least one exchange, so that no tile writes its result
+// before its neighbours have read their inputs; an image of a single tile needs none.
+static hs_status launch_table(ResidentTable &tab, int r, bool zero_start, const ResolvedConfig &rc, cudaStream_t s) {
     tab.first[0] = 0;
     bool several = false;
     for (int i = 0; i < tab.n; ++i) {
-        const int tiles = tab.img[i].ntx * tab.img[i].nty;
+        ResImage &p = tab.img[i];
+        const int tiles = p.ntx * p.nty;
         tab.first[i + 1] = tab.first[i] + tiles;
         several |= tiles > 1;
+        p.nblocks = tiles > 1 ? std::max(2, (p.iters + kResT - 1) / kResT) : 1;
     }
     tab.we = rc.we;
     tab.wc = rc.wc;
-    tab.iters = iters;
-    tab.nblocks = several ? std::max(2, (iters + kResT - 1) / kResT) : 1;
     tab.zero_start = zero_start ? 1 : 0;
+    if (several && tab.n == 1) {  // the flag lies behind the one image's outboxes
+        const size_t bytes = resident_box_bytes(tab.first[1], r);
+        HS_CUDA_CHECK(cudaMemsetAsync(tab.img[0].box, 0, bytes, s));
+    } else if (several) {
+        res_clear_kernel<<<tab.first[tab.n], 256, 0, s>>>(tab, res_msgs(kResWarps * r));
+        HS_LAUNCH_CHECK("res_clear_kernel");
+    }
     switch (r) {
 #define HS_RES(RR) \
     case RR: return rc.fast ? launch_resident<true, kResWarps, RR>(tab, s) : launch_resident<false, kResWarps, RR>(tab, s);
@@ -441,69 +465,76 @@ hs_status run_resident(const float *I0, const float *I1, const float *Ix, const 
     p.H = H; p.W = W; p.ld = ld;
     p.alpha2 = alpha2;
     p.ntx = pl.ntx; p.nty = pl.nty;
-    if (pl.box_bytes) {
-        HS_CUDA_CHECK(cudaMemsetAsync(scratch, 0, pl.box_bytes, s));
+    p.iters = iters;
+    if (pl.box_bytes)
         tab.abort_flag = reinterpret_cast<unsigned *>(reinterpret_cast<char *>(scratch) + pl.box_bytes - 256);
-    }
-    return launch_table(tab, pl.r, iters, zero_start, rc, s);
+    return launch_table(tab, pl.r, zero_start, rc, s);
 }
 
 // ---- many images: groups whose tiles the SMs hold all at once, one launch each
 
-// Greedy groups in order with r rows per warp; returns their number, 0 if an image does not fit.
-static int resident_groups(const ResidentJob *jobs, int n, int r, int *group_end) {
-    int groups = 0, tiles = 0;
-    for (int i = 0; i < n; ++i) {
-        int ntx, nty;
-        const int t = resident_tiles(jobs[i].H, jobs[i].W, r, &ntx, &nty);
-        if (t > sm_count() || resident_box_bytes(t, r) > jobs[i].scratch_bytes) return 0;
-        if (tiles + t > sm_count()) {
-            group_end[groups++] = i;
-            tiles = 0;
+// How the jobs, in their order, are cut into launches: launch k holds jobs end[k-1] .. end[k]-1
+// with r[k] rows per warp.  A launch takes as long as its longest image, and a sweep of it about
+// 0.65 + 0.22 r us in the fast form, 0.5 + 0.52 r in the exact one, whatever the number of tiles
+// (measured at 320x240 .. 1920x1080, r = 2 .. 8): tall tiles put more images into a launch, low
+// ones spread an image over more SMs.  The cut that needs the least time in all (dynamic
+// programming over the prefixes).  false if an image does not fit.
+struct ResidentCut {
+    std::vector<int> end, r;
+};
+static bool resident_cut(const ResidentJob *jobs, int n, bool fast, ResidentCut &cut) {
+    std::vector<double> cost(n + 1, -1.0);
+    std::vector<int> from(n + 1, 0), rows(n + 1, 0);
+    cost[0] = 0.0;
+    for (int i = 0; i < n; ++i) {  // a launch that starts with job i
+        if (cost[i] < 0.0) continue;
+        for (int r = kResMinR; r <= kResMaxR; ++r) {
+            const double sweep = fast ? 0.65 + 0.22 * r : 0.5 + 0.52 * r;
+            int tiles = 0, longest = 0;
+            for (int j = i; j < n && j < i + kMaxResImages; ++j) {
+                int ntx, nty;
+                const int t = resident_tiles(jobs[j].H, jobs[j].W, r, &ntx, &nty);
+                tiles = std::min(tiles + std::min(t, sm_count() + 1), sm_count() + 1);
+                if (tiles > sm_count() || resident_box_bytes(t, r) > jobs[j].scratch_bytes) break;
+                longest = std::max(longest, jobs[j].iters);
+                const double c = cost[i] + sweep * longest + 8.0;  // (and about 8 us for a launch)
+                if (cost[j + 1] < 0.0 || c < cost[j + 1]) {
+                    cost[j + 1] = c;
+                    from[j + 1] = i;
+                    rows[j + 1] = r;
+                }
+            }
         }
-        tiles += t;
     }
-    group_end[groups++] = n;
-    return groups;
+    if (cost[n] < 0.0) return false;
+    cut.end.clear();
+    cut.r.clear();
+    for (int j = n; j > 0; j = from[j]) {
+        cut.end.insert(cut.end.begin(), j);
+        cut.r.insert(cut.r.begin(), rows[j]);
+    }
+    return true;
 }
 
-// A sweep of one launch takes about 0.9 + 0.2 r us in the fast form (1080p, 1.9 x the slope in the
-// exact form), whatever the number of tiles; the tile height that needs the least in all.
-int resident_choose(const ResidentJob *jobs, int n, bool fast, int *group_end) {
-    int best_r = 0;
-    double best = 0.0;
-    int ends[kMaxResImages];
-    for (int r = kResMinR; r <= kResMaxR; ++r) {
-        const int g = resident_groups(jobs, n, r, ends);
-        if (g == 0) continue;
-        const double cost = g * (0.9 + (fast ? 0.2 : 0.38) * r);
-        if (best_r == 0 || cost < best) {
-            best_r = r;
-            best = cost;
-        }
-    }
-    if (best_r) resident_groups(jobs, n, best_r, group_end);
-    return best_r;
+bool resident_fits(int H, int W, int iters, size_t scratch_bytes) {
+    ResidentPlan pl;
+    return resident_plan(H, W, iters, scratch_bytes, pl);
 }
 
-hs_status run_resident_jobs(const ResidentJob *jobs, int n, int iters, int ckpt_every, size_t ckpt_plane,
+hs_status run_resident_jobs(const ResidentJob *jobs, int n, int ckpt_every, size_t ckpt_plane, int *status,
                             const ResolvedConfig &rc, cudaStream_t s) {
-    int ends[kMaxResImages];
-    if (n > kMaxResImages || iters < 2) return HS_ERR_UNSUPPORTED;
-    if (resident_choose(jobs, n, rc.fast, ends) == 0) return HS_ERR_UNSUPPORTED;
-    for (int i0 = 0, g = 0; i0 < n; i0 = ends[g++]) {
-        const int m = ends[g] - i0;
-        int sub[kMaxResImages];
-        // (a last, smaller group may take smaller tiles)
-        int r = 0;
-        for (int q = kResMinR; q <= kResMaxR && !r; ++q)
-            if (resident_groups(jobs + i0, m, q, sub) == 1) r = q;
+    for (int i = 0; i < n; ++i)
+        if (jobs[i].iters < 2) return HS_ERR_UNSUPPORTED;
+    ResidentCut cut;
+    if (!resident_cut(jobs, n, rc.fast, cut)) return HS_ERR_UNSUPPORTED;
+    for (size_t g = 0; g < cut.end.size(); ++g) {
+        const int i0 = g ? cut.end[g - 1] : 0, m = cut.end[g] - i0, r = cut.r[g];
         ResidentTable tab;
         memset(&tab, 0, sizeof(tab));
         tab.n = m;
         tab.ckpt_every = ckpt_every;
         tab.ckpt_plane = ckpt_plane;
-        size_t box = 0;
+        tab.status = status;
         for (int i = 0; i < m; ++i) {
             const ResidentJob &d = jobs[i0 + i];
             ResImage &p = tab.img[i];
@@ -513,21 +544,14 @@ hs_status run_resident_jobs(const ResidentJob *jobs, int n, int iters, int ckpt_
             p.ckpt = d.ckpt;
             p.box = reinterpret_cast<float4 *>(d.scratch);
             p.alpha_dev = d.alpha_dev;
+            p.alpha2 = d.alpha2;
             p.H = d.H; p.W = d.W; p.ld = d.ld;
+            p.iters = d.iters;
             const int tiles = resident_tiles(d.H, d.W, r, &p.ntx, &p.nty);
-            const size_t bytes = resident_box_bytes(tiles, r);
-            if (bytes > box) {
-                box = bytes;
-                tab.abort_flag = reinterpret_cast<unsigned *>(d.scratch + bytes - 256);
-            }
+            if (tiles > 1)
+                tab.abort_flag = reinterpret_cast<unsigned *>(d.scratch + resident_box_bytes(tiles, r) - 256);
         }
-        // clear the outboxes: the jobs' scratch buffers lie one stride apart
-        if (box && m == 1) HS_CUDA_CHECK(cudaMemsetAsync(jobs[i0].scratch, 0, box, s));
-        if (box && m > 1) {
-            const size_t pitch = jobs[i0 + 1].scratch - jobs[i0].scratch;
-            HS_CUDA_CHECK(cudaMemset2DAsync(jobs[i0].scratch, pitch, 0, box, m, s));
-        }
-        const hs_status st = launch_table(tab, r, iters, true, rc, s);
+        const hs_status st = launch_table(tab, r, true, rc, s);
         if (st != HS_OK) return st;
     }
     return HS_OK;

@@ -60,17 +60,18 @@ struct ResImage {
     float alpha2;
     int H, W, ld;
     int ntx, nty;                // tiles across and down
+    int iters, nblocks;          // the sweeps run in nblocks blocks of at most kResT
 };
 
 struct ResidentTable {
     ResImage img[kMaxResImages];
     int first[kMaxResImages + 1];  // tiles of the images before image i
     int n;
-    unsigned *abort_flag;
+    unsigned *abort_flag;        // raised by a wait that ran out
+    int *status;                 // if set: HS_ERR_TIMEOUT goes here then
     size_t ckpt_plane;           // floats between checkpoint planes
     int ckpt_every;
     float we, wc;
-    int iters, nblocks;          // the sweeps run in nblocks blocks of at most kResT
     int zero_start;
 };
 

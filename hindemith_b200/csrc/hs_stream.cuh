@@ -434,19 +434,23 @@ bool resident_plan(int H, int W, int iters, size_t scratch_bytes, ResidentPlan &
 hs_status run_resident(const float *I0, const float *I1, const float *Ix, const float *Iy, const float *It, int H,
                        int W, int ld, float alpha2, int iters, float *u, float *v, void *scratch, bool zero_start,
                        const ResolvedConfig &rc, const ResidentPlan &pl, cudaStream_t s);
-// The resident form for many images (training): derivatives into Ix, Iy, It, the state after
-// every ckpt_every sweeps into the checkpoint planes (ckpt_plane floats apart; u then v), the
-// final state into u, v as well.  The jobs' scratch buffers have one size and lie one stride
-// apart.  HS_ERR_UNSUPPORTED when an image does not fit (any launches made are to be redone).
+// Whether an image can run in the resident form.
+bool resident_fits(int H, int W, int iters, size_t scratch_bytes);
+// The resident form for many images, each with its own size and sweeps (>= 2), in launches of as
+// many as fit the chip at once; the flow goes to u, v.  Training: derivatives into Ix, Iy, It (may
+// be null), the state after every ckpt_every sweeps into the checkpoint planes (ckpt_plane floats
+// apart; u then v).  status, if set, receives HS_ERR_TIMEOUT when a wait runs out.
+// HS_ERR_UNSUPPORTED when an image does not fit (any launches made are to be redone).
 struct ResidentJob {
     const float *I0, *I1;
     float *Ix, *Iy, *It, *u, *v, *ckpt;
-    char *scratch;
+    char *scratch;  // 16-byte aligned
     size_t scratch_bytes;
-    const float *alpha_dev;
-    int H, W, ld;
+    const float *alpha_dev;  // or alpha2 when null
+    float alpha2;
+    int H, W, ld, iters;
 };
-hs_status run_resident_jobs(const ResidentJob *jobs, int n, int iters, int ckpt_every, size_t ckpt_plane,
+hs_status run_resident_jobs(const ResidentJob *jobs, int n, int ckpt_every, size_t ckpt_plane, int *status,
                             const ResolvedConfig &rc, cudaStream_t s);
 // A depth, a segment size or a layout in hs_config asks for the streaming passes.
 inline bool wants_resident(const ResolvedConfig &rc) { return rc.T_default && rc.seg_rows == 0 && rc.layout == 0; }

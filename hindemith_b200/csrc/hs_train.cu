@@ -721,9 +721,9 @@ static hs_status train_forward(const hs_train_pair *pairs, const PairBufs *bufs,
             const hs_train_pair &d = pairs[i];
             const PairBufs &B = bufs[i];
             jobs[i] = {d.I0, d.I1, B.deriv(0), B.deriv(1), B.deriv(2), d.u, d.v, B.ck(0, 0), B.scratch,
-                       4 * B.pb, d.alpha, d.H, d.W, d.ld};
+                       4 * B.pb, d.alpha, 0.f, d.H, d.W, d.ld, iters};
         }
-        st = run_resident_jobs(jobs.data(), n, iters, ckpt_every, bufs[0].pb / sizeof(float), rc, s);
+        st = run_resident_jobs(jobs.data(), n, ckpt_every, bufs[0].pb / sizeof(float), nullptr, rc, s);
         if (st != HS_ERR_UNSUPPORTED) return st;
     }
     for (int i = 0; i < n; ++i) {

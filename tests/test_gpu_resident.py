@@ -170,3 +170,19 @@ def test_wide_passes_with_the_ring_in_tensor_memory(cuda, shape, T):
         D.hs_sweeps(Ix, Iy, It, 0.3, 2 * T + 1, *pair, L.make_config(fast_math=True, sweeps_per_pass=T, layout=layout))
     same(got[0], ref[0], "u")
     same(got[1], ref[1], "v")
+
+
+@pytest.mark.parametrize("scale", [1e-30, 1e-20, 1e-12, 1e-6, 1.0, 1e6, 1e12, 1e18])
+@pytest.mark.parametrize("alpha", [0.0, 1e-18, 1e-7, 1e-3, 1.0, 1e6, 1e12])
+def test_resident_exact_division_over_the_float_range(cuda, scale, alpha):
+    """The exact form's quotient equals the IEEE division of the streaming passes wherever its
+    numerators and denominators lie: tiny, huge, zero and non-finite ones included."""
+    I0, I1 = planes((70, 260), 2, seed=7)
+    I0, I1 = D.as_plane(I0 * scale), D.as_plane(I1 * scale)
+    I0[30:40, 50:90] = 0.5 * scale  # a flat patch: zero derivatives
+    I1[30:40, 50:90] = 0.5 * scale
+    with np.errstate(all="ignore"):
+        u, v = D.hs_forward(I0, I1, alpha, 13)
+        ru, rv = D.hs_forward(I0, I1, alpha, 13, L.make_config(sweeps_per_pass=2, layout=1))
+    same(u, ru, "u")
+    same(v, rv, "v")

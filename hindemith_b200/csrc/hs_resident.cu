@@ -20,53 +20,6 @@
 
 namespace hs {
 
-// Polls of one message, at most: a few seconds.  A wait can only run out if a neighbour's CTA
-// has stopped (all CTAs of the cooperative launch are resident together); the tile then raises
-// the abort flag, stops waiting, and the tiles that see the flag write NaN as their result.
-constexpr int kResPolls = 1 << 22;
-
-// One 128-bit access of a message (single-copy atomic).
-__device__ __forceinline__ void msg_store(float4 *p, float a, float b, float c, unsigned e) {
-    asm volatile(
-        "{\n\t.reg .b128 q;\n\t.reg .b64 lo, hi;\n\t"
-        "mov.b64 lo, {%1, %2};\n\tmov.b64 hi, {%3, %4};\n\tmov.b128 q, {lo, hi};\n\t"
-        "st.relaxed.gpu.global.b128 [%0], q;\n\t}" ::"l"(p), "f"(a), "f"(b), "f"(c), "r"(e)
-        : "memory");
-}
-__device__ __forceinline__ void msg_load(const float4 *p, float (&f)[3], unsigned &e) {
-    asm volatile(
-        "{\n\t.reg .b128 q;\n\t.reg .b64 lo, hi;\n\t"
-        "ld.relaxed.gpu.global.b128 q, [%4];\n\tmov.b128 {lo, hi}, q;\n\t"
-        "mov.b64 {%0, %1}, lo;\n\tmov.b64 {%2, %3}, hi;\n\t}"
-        : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=r"(e)
-        : "l"(p)
-        : "memory");
-}
-
-// A chunk (8 floats, 16-byte aligned) to and from the lane's columns of a row.
-__device__ __forceinline__ void put_chunk(float *s, const float2 (&c)[2][2]) {
-    reinterpret_cast<float4 *>(s)[0] = cat4(c[0][0], c[0][1]);
-    reinterpret_cast<float4 *>(s)[1] = cat4(c[1][0], c[1][1]);
-}
-__device__ __forceinline__ void get_chunk(const float *s, float2 (&c)[2][2]) {
-    const float4 u = reinterpret_cast<const float4 *>(s)[0], v = reinterpret_cast<const float4 *>(s)[1];
-    c[0][0] = lo2(u);
-    c[0][1] = hi2(u);
-    c[1][0] = lo2(v);
-    c[1][1] = hi2(v);
-}
-
-// Shared memory of a CTA: the sweeps' publications, the chunks sent, the chunks received and,
-// for every message received, where it comes from.
-template <int NW, int R>
-struct ResSmem {
-    static constexpr int chunks = res_chunks(NW * R), msgs = res_msgs(NW * R);
-    static constexpr int out = 2 * NW * 128 * 16;        // bytes
-    static constexpr int in = out + chunks * 32 + 16;    // (a chunk's third message reads 1 float past it)
-    static constexpr int src = in + chunks * 32 + 16;
-    static constexpr int bytes = src + msgs * 4;
-};
-
 template <bool FAST, int NW, int R>
 __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_constant__ ResidentTable tab) {
     using S = ResSmem<NW, R>;
@@ -87,26 +40,13 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
     int image = 0;
     while (image + 1 < tab.n && tab.first[image + 1] <= (int)blockIdx.x) ++image;
     const ResImage &p = tab.img[image];
-    const int tile = blockIdx.x - tab.first[image], tx = tile % p.ntx, ty = tile / p.ntx;
+    const int tile = blockIdx.x - tab.first[image];
     const float alpha2 = p.alpha_dev ? __fmul_rn(__ldg(p.alpha_dev), __ldg(p.alpha_dev)) : p.alpha2;
-    const int chunks = (p.W + 3) / 4;
-    const int x0 = 4 * res_split(tx, p.ntx, chunks), x1 = 4 * res_split(tx + 1, p.ntx, chunks);
-    const int y0 = res_split(ty, p.nty, p.H), y1 = res_split(ty + 1, p.nty, p.H);
-    const int xa = x0 - 4 + 4 * lane;  // the lane's first column (a multiple of 4)
-    const int own = (x1 - x0) / 4;     // lanes 1 .. own hold the tile's own columns
-
     ResLane t;
-    t.lane = lane;
-    t.warp = warp;
-    t.first = xa == 0;
-    t.last = xa <= p.W - 1 && xa + 4 > p.W - 1;
-    t.row0 = y0 - kResT + warp * R;
-    t.H = p.H;
-    t.tmem = tmem + ((unsigned)(warp & 3) << 21) + (unsigned)(warp >> 2) * (R * 16);
-    // every plane row holds whole chunks (ld % 4 == 0), so a chunk that starts inside the image
-    // may be read; other chunks are never needed
-    const bool col_in = xa >= 0 && xa < p.W;
-    const bool own_col = lane >= 1 && lane <= own;
+    ResTile g;
+    res_tile<R>(g, t, tile, p.ntx, p.nty, p.H, p.W, p.ld, tmem);
+    const int xa = g.xa;
+    const bool col_in = g.col_in;
 
     // start state and coefficients
     float2 cu[R][2][2];
@@ -142,7 +82,7 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
                 const float b[4] = {i1[j], i1[j + 1], n1[j], n1[j + 1]};
                 hs_derivs_taps(a, b, c[j], c[4 + j], c[8 + j]);
             }
-            if (p.Ix && own_col && row >= y0 && row < y1) {  // (scratch planes: whole chunks)
+            if (p.Ix && g.own_col && row >= g.y0 && row < g.y1) {  // (scratch planes: whole chunks)
                 *reinterpret_cast<float4 *>(p.Ix + off) = make_float4(c[0], c[1], c[2], c[3]);
                 *reinterpret_cast<float4 *>(p.Iy + off) = make_float4(c[4], c[5], c[6], c[7]);
                 *reinterpret_cast<float4 *>(p.It + off) = make_float4(c[8], c[9], c[10], c[11]);
@@ -177,156 +117,32 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
     __threadfence();
     __syncwarp();
 
-    const bool nl = tx > 0, nr = tx + 1 < p.ntx, nu = ty > 0, nd = ty + 1 < p.nty;
-    const int side = nl && nr ? -1 : (p.W - 1) & 3;
-    const bool ghosts = (t.row0 < 0 && t.row0 + R > 0) || (t.row0 < p.H && t.row0 + R > p.H);
-    // where each message received comes from: its index in all outboxes' first half, -1: none
-    const int half_msgs = p.ntx * p.nty * S::msgs;
-    if (p.nblocks > 1) {
-        const int lown = nl ? res_split(tx, p.ntx, chunks) - res_split(tx - 1, p.ntx, chunks) : 0;
-        for (int i = threadIdx.x; i < S::msgs; i += NW * 32) {
-            const int c = i / 3, m = i % 3;
-            int dx = 0, dy = 0, from = -1;  // the neighbour and its chunk
-            if (c < 2 * kResRowChunks) {
-                const int blk = c / kResRowChunks, l = c % 32;  // 0: above, from that tile's last rows
-                dy = blk == 0 ? -1 : 1;
-                dx = l == 0 ? -1 : l == own + 1 ? 1 : 0;
-                if (l <= own + 1)
-                    from = (1 - blk) * kResRowChunks + (c % kResRowChunks) - l + (l == 0 ? lown : l == own + 1 ? 1 : l);
-            } else {
-                const int k = c - 2 * kResRowChunks, sd = k >= NW * R, lr = k - sd * (NW * R);
-                dx = sd ? 1 : -1;
-                const int row = y0 - kResT + lr;
-                if (row >= y0 && row < y1) from = 2 * kResRowChunks + (1 - sd) * (NW * R) + lr;
-            }
-            const int nx = tx + dx, ny = ty + dy;
-            if (nx < 0 || nx >= p.ntx || ny < 0 || ny >= p.nty) from = -1;
-            src[i] = from < 0 ? -1 : (ny * p.ntx + nx) * S::msgs + 3 * from + m;
-        }
-        // chunks that nobody sends stay 0: cells that are never used, but garbage there (a NaN)
-        // would send whole warps through the exact form's general division
-        for (int i = threadIdx.x; i < S::chunks * 8; i += NW * 32) in[i] = 0.f;
-    }
-    // (uniform in the warp) rows of the ring, and rows of the halo, among the warp's
-    const int row_end = t.row0 + R;
-    const bool up_rows = t.row0 < y0 + kResT && row_end > y0, down_rows = t.row0 < y1 && row_end > y1 - kResT;
-    const bool above_rows = t.row0 < y0, below_rows = t.row0 < y1 + kResT && row_end > y1;
-    // the tile's own pixels of the state to planes U, V
-    auto store_own = [&](float *U, float *V) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int row = t.row0 + r;
-            if (row >= y0 && row < y1 && own_col) res_store(U, V, (size_t)row * p.ld + xa, p.W - xa, cu[r]);
-        }
-        __syncwarp();
-    };
-    if (p.ckpt) store_own(p.ckpt, p.ckpt + tab.ckpt_plane);  // checkpoint 0: the start state
+    if (p.nblocks > 1) res_sources<NW, R>(g, src, in);
+    bool ok = true;
+    if (p.ckpt) res_store_own<R>(t, g, cu, p.ckpt, p.ckpt + tab.ckpt_plane);  // checkpoint 0: the start state
     int done = 0, ck = 1;  // ck: the next checkpoint
     for (int b = 0; b < p.nblocks; ++b) {
         const int upto = res_split(b + 1, p.nblocks, p.iters);
         while (done < upto) {
             const int next = p.ckpt ? min(upto, ck * tab.ckpt_every) : upto, n = next - done;
-            // (uniform in the CTA; every variant runs one block barrier per sweep)
-            switch (side) {
-                case -1: res_sweeps<FAST, NW, R, -1>(t, cu, pub, done & 1, n, ghosts, tab.we, tab.wc); break;
-                case 0: res_sweeps<FAST, NW, R, 0>(t, cu, pub, done & 1, n, ghosts, tab.we, tab.wc); break;
-                case 1: res_sweeps<FAST, NW, R, 1>(t, cu, pub, done & 1, n, ghosts, tab.we, tab.wc); break;
-                case 2: res_sweeps<FAST, NW, R, 2>(t, cu, pub, done & 1, n, ghosts, tab.we, tab.wc); break;
-                default: res_sweeps<FAST, NW, R, 3>(t, cu, pub, done & 1, n, ghosts, tab.we, tab.wc); break;
-            }
+            res_run<FAST, NW, R>(t, g, cu, pub, done & 1, n, tab.we, tab.wc);
             done = next;
             if (p.ckpt && (done == ck * tab.ckpt_every || done == p.iters)) {
-                store_own(p.ckpt + (size_t)(2 * ck) * tab.ckpt_plane, p.ckpt + (size_t)(2 * ck + 1) * tab.ckpt_plane);
+                res_store_own<R>(t, g, cu, p.ckpt + (size_t)(2 * ck) * tab.ckpt_plane,
+                                 p.ckpt + (size_t)(2 * ck + 1) * tab.ckpt_plane);
                 ++ck;
             }
         }
         if (b + 1 == p.nblocks) break;
         if (p.ntx * p.nty == 1) continue;  // no neighbours
 
-        // exchange e: the ring into shared memory
-        const unsigned e = (unsigned)(b + 1);
-        if ((lane == 1 && nl) || (lane == own && nr)) {  // (own >= 2 in a tile with neighbours beside it)
-            float *f = out + 8 * (2 * kResRowChunks + (lane == 1 ? 0 : NW * R) + warp * R);
-#pragma unroll
-            for (int r = 0; r < R; ++r) put_chunk(f + 8 * r, cu[r]);
+        if (!res_exchange<NW, R, false>(t, g, cu, out, in, src, p.box, (unsigned)(b + 1), &stop, tab.abort_flag,
+                                        tab.status)) {
+            ok = false;
+            break;
         }
-        if (up_rows || down_rows) {
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const int j = t.row0 + r - y0, k = t.row0 + r - (y1 - kResT);
-                if (j >= 0 && j < kResT) put_chunk(out + 8 * (32 * j + lane), cu[r]);
-                if (k >= 0 && k < kResT) put_chunk(out + 8 * (kResRowChunks + 32 * k + lane), cu[r]);
-            }
-        }
-        __syncthreads();
-        float4 *boxes = p.box + ((e & 1u) ? (size_t)half_msgs : 0);
-        float4 *mine = boxes + (size_t)tile * S::msgs;
-        constexpr int kPer = (S::msgs + NW * 32 - 1) / (NW * 32);  // messages per thread
-#pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-            const int m = threadIdx.x + i * NW * 32;
-            if (m < S::msgs) {
-                const float *f = out + 8 * (m / 3) + 3 * (m % 3);
-                msg_store(mine + m, f[0], f[1], f[2], e);
-            }
-        }
-        // receive: all of the thread's loads in flight, until each carries e
-        int from[kPer];
-        float got[kPer][3];
-        unsigned tag[kPer];
-#pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-            const int m = threadIdx.x + i * NW * 32;
-            from[i] = m < S::msgs ? src[m] : -1;
-            tag[i] = e;
-            if (from[i] >= 0) msg_load(boxes + from[i], got[i], tag[i]);
-        }
-        for (int polls = 0;;) {
-            bool all = true;
-#pragma unroll
-            for (int i = 0; i < kPer; ++i) all = all && tag[i] == e;
-            if (all) break;
-            if (++polls > kResPolls ||
-                ((polls & 1023) == 0 && (*(volatile int *)&stop || *(volatile unsigned *)tab.abort_flag))) {
-                atomicExch(tab.abort_flag, 1u);
-                if (tab.status) atomicCAS(tab.status, 0, (int)HS_ERR_TIMEOUT);
-                *(volatile int *)&stop = 1;
-                break;
-            }
-#pragma unroll
-            for (int i = 0; i < kPer; ++i)
-                if (tag[i] != e) msg_load(boxes + from[i], got[i], tag[i]);
-        }
-#pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-            const int m = threadIdx.x + i * NW * 32;
-            if (from[i] >= 0) {
-                float *f = in + 8 * (m / 3) + 3 * (m % 3);
-                f[0] = got[i][0];
-                f[1] = got[i][1];
-                if (m % 3 < 2) f[2] = got[i][2];
-            }
-        }
-        __syncthreads();
-        if (stop) break;
-        if ((lane == 0 && nl) || (lane == own + 1 && nr)) {
-            const float *f = in + 8 * (2 * kResRowChunks + (lane == 0 ? 0 : NW * R) + warp * R);
-#pragma unroll
-            for (int r = 0; r < R; ++r) get_chunk(f + 8 * r, cu[r]);
-        }
-        if ((above_rows && nu) || (below_rows && nd)) {
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const int j = t.row0 + r - (y0 - kResT), k = t.row0 + r - y1;
-                if (nu && j < kResT) get_chunk(in + 8 * (32 * j + lane), cu[r]);
-                if (nd && k >= 0 && k < kResT) get_chunk(in + 8 * (kResRowChunks + 32 * k + lane), cu[r]);
-            }
-        }
-        __syncwarp();
     }
-    __syncthreads();
-    bool ok = true;
-    if (p.nblocks > 1) ok = stop == 0 && *(volatile unsigned *)tab.abort_flag == 0u;
+    if (p.nblocks > 1) ok = ok && *(volatile unsigned *)tab.abort_flag == 0u;
     if (!ok) {
         const float2 nan2 = f2(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
 #pragma unroll
@@ -334,7 +150,7 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
 #pragma unroll
             for (int q = 0; q < 2; ++q) cu[r][q][0] = cu[r][q][1] = nan2;
     }
-    store_own(p.u, p.v);
+    res_store_own<R>(t, g, cu, p.u, p.v);
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, kCols);
 }
@@ -474,22 +290,18 @@ hs_status run_resident(const float *I0, const float *I1, const float *Ix, const 
 // ---- many images: groups whose tiles the SMs hold all at once, one launch each
 
 // How the jobs, in their order, are cut into launches: launch k holds jobs end[k-1] .. end[k]-1
-// with r[k] rows per warp.  A launch takes as long as its longest image, and a sweep of it about
-// 0.65 + 0.22 r us in the fast form, 0.5 + 0.52 r in the exact one, whatever the number of tiles
-// (measured at 320x240 .. 1920x1080, r = 2 .. 8): tall tiles put more images into a launch, low
+// with r[k] rows per warp.  A launch takes as long as its longest image, and a sweep of it
+// base + slope * r us, whatever the number of tiles: tall tiles put more images into a launch, low
 // ones spread an image over more SMs.  The cut that needs the least time in all (dynamic
 // programming over the prefixes).  false if an image does not fit.
-struct ResidentCut {
-    std::vector<int> end, r;
-};
-static bool resident_cut(const ResidentJob *jobs, int n, bool fast, ResidentCut &cut) {
+bool resident_cut(const ResidentJob *jobs, int n, double base, double slope, int max_r, ResidentCut &cut) {
     std::vector<double> cost(n + 1, -1.0);
     std::vector<int> from(n + 1, 0), rows(n + 1, 0);
     cost[0] = 0.0;
     for (int i = 0; i < n; ++i) {  // a launch that starts with job i
         if (cost[i] < 0.0) continue;
-        for (int r = kResMinR; r <= kResMaxR; ++r) {
-            const double sweep = fast ? 0.65 + 0.22 * r : 0.5 + 0.52 * r;
+        for (int r = kResMinR; r <= max_r; ++r) {
+            const double sweep = base + slope * r;
             int tiles = 0, longest = 0;
             for (int j = i; j < n && j < i + kMaxResImages; ++j) {
                 int ntx, nty;
@@ -526,7 +338,8 @@ hs_status run_resident_jobs(const ResidentJob *jobs, int n, int ckpt_every, size
     for (int i = 0; i < n; ++i)
         if (jobs[i].iters < 2) return HS_ERR_UNSUPPORTED;
     ResidentCut cut;
-    if (!resident_cut(jobs, n, rc.fast, cut)) return HS_ERR_UNSUPPORTED;
+    // us per sweep, measured at 320x240 .. 1920x1080, r = 2 .. 8
+    if (!resident_cut(jobs, n, rc.fast ? 0.65 : 0.5, rc.fast ? 0.22 : 0.52, kResMaxR, cut)) return HS_ERR_UNSUPPORTED;
     for (size_t g = 0; g < cut.end.size(); ++g) {
         const int i0 = g ? cut.end[g - 1] : 0, m = cut.end[g] - i0, r = cut.r[g];
         ResidentTable tab;

@@ -189,7 +189,8 @@ __device__ __forceinline__ void res_barrier() { asm volatile("bar.sync 0;" ::: "
 //   fast : the first and the last row's Y
 //   exact: the first row itself (its three lower taps are added one by one) and the last
 //          row's `up`
-template <bool FAST, int NW, int R, int SIDE>
+// UPDATE = false: only the average, A (the adjoint's use).
+template <bool FAST, int NW, int R, int SIDE, bool UPDATE = true>
 __device__ __forceinline__ void res_sweep(const ResLane &t, float2 (&cu)[R][2][2], float4 *pub, float wef,
                                           float wcf) {
     const float2 we = f2(wef, wef), wc = f2(wcf, wcf);
@@ -233,7 +234,7 @@ __device__ __forceinline__ void res_sweep(const ResLane &t, float2 (&cu)[R][2][2
         }
     }
     float co[16];
-    tmem_ld16(co, t.tmem);
+    if constexpr (UPDATE) tmem_ld16(co, t.tmem);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         // terms of row r + 1
@@ -269,16 +270,23 @@ __device__ __forceinline__ void res_sweep(const ResLane &t, float2 (&cu)[R][2][2
                     if (r + 1 < R) acc[q][j] = add2(add2(cur[q][j].up, nxt[q][j].ml), nxt[q][j].mr);
                 }
             }
-        tmem_wait_ld(co);
-        float cn[16];
+        if constexpr (UPDATE) {
+            tmem_wait_ld(co);
+            float cn[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) cn[i] = co[i];
-        if (r + 1 < R) tmem_ld16(co, t.tmem + 16 * (r + 1));
+            for (int i = 0; i < 16; ++i) cn[i] = co[i];
+            if (r + 1 < R) tmem_ld16(co, t.tmem + 16 * (r + 1));
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
-            res_update<FAST>(avg[0][j], avg[1][j], f2(cn[2 * j], cn[2 * j + 1]), f2(cn[4 + 2 * j], cn[5 + 2 * j]),
-                             f2(cn[8 + 2 * j], cn[9 + 2 * j]), f2(cn[12 + 2 * j], cn[13 + 2 * j]), cu[r][0][j],
-                             cu[r][1][j]);
+            for (int j = 0; j < 2; ++j)
+                res_update<FAST>(avg[0][j], avg[1][j], f2(cn[2 * j], cn[2 * j + 1]), f2(cn[4 + 2 * j], cn[5 + 2 * j]),
+                                 f2(cn[8 + 2 * j], cn[9 + 2 * j]), f2(cn[12 + 2 * j], cn[13 + 2 * j]), cu[r][0][j],
+                                 cu[r][1][j]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) cu[r][q][j] = avg[q][j];
+        }
 #pragma unroll
         for (int q = 0; q < 2; ++q)
 #pragma unroll
@@ -312,13 +320,13 @@ __device__ __forceinline__ void res_ghost_rows(const ResLane &t, float2 (&cu)[R]
 // n sweeps of the warp's rows; pub: both halves of the publication buffer, `half` the one to use.
 // (The loop is inside the variant: its state registers need not agree with another variant's
 // after every sweep.)
-template <bool FAST, int NW, int R, int SIDE>
+template <bool FAST, int NW, int R, int SIDE, bool UPDATE = true>
 __device__ __forceinline__ void res_sweeps(const ResLane &t, float2 (&cu)[R][2][2], float4 *pub, int half, int n,
                                            bool ghosts, float wef, float wcf) {
 #pragma unroll 1
     for (int i = 0; i < n; ++i, half ^= 1) {
         if (ghosts) res_ghost_rows<R>(t, cu);
-        res_sweep<FAST, NW, R, SIDE>(t, cu, pub + half * (NW * 128), wef, wcf);
+        res_sweep<FAST, NW, R, SIDE, UPDATE>(t, cu, pub + half * (NW * 128), wef, wcf);
     }
 }
 
@@ -369,6 +377,254 @@ constexpr int res_tmem_cols() {
     constexpr int words = (NW / 4) * R * 16;
     static_assert(NW % 4 == 0 && words <= 512, "the coefficients of a tile fit tensor memory");
     return words <= 32 ? 32 : words <= 64 ? 64 : words <= 128 ? 128 : words <= 256 ? 256 : 512;
+}
+
+// Polls of one message, at most: a few seconds.  A wait can only run out if a neighbour's CTA
+// has stopped (all CTAs of the cooperative launch are resident together); the tile then raises
+// the abort flag, stops waiting, and the tiles that see the flag write NaN as their result.
+constexpr int kResPolls = 1 << 22;
+
+// One 128-bit access of a message (single-copy atomic).
+__device__ __forceinline__ void msg_store(float4 *p, float a, float b, float c, unsigned e) {
+    asm volatile(
+        "{\n\t.reg .b128 q;\n\t.reg .b64 lo, hi;\n\t"
+        "mov.b64 lo, {%1, %2};\n\tmov.b64 hi, {%3, %4};\n\tmov.b128 q, {lo, hi};\n\t"
+        "st.relaxed.gpu.global.b128 [%0], q;\n\t}" ::"l"(p), "f"(a), "f"(b), "f"(c), "r"(e)
+        : "memory");
+}
+__device__ __forceinline__ void msg_load(const float4 *p, float (&f)[3], unsigned &e) {
+    asm volatile(
+        "{\n\t.reg .b128 q;\n\t.reg .b64 lo, hi;\n\t"
+        "ld.relaxed.gpu.global.b128 q, [%4];\n\tmov.b128 {lo, hi}, q;\n\t"
+        "mov.b64 {%0, %1}, lo;\n\tmov.b64 {%2, %3}, hi;\n\t}"
+        : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=r"(e)
+        : "l"(p)
+        : "memory");
+}
+
+// A chunk (8 floats, 16-byte aligned) to and from the lane's columns of a row.
+__device__ __forceinline__ void put_chunk(float *s, const float2 (&c)[2][2]) {
+    reinterpret_cast<float4 *>(s)[0] = cat4(c[0][0], c[0][1]);
+    reinterpret_cast<float4 *>(s)[1] = cat4(c[1][0], c[1][1]);
+}
+__device__ __forceinline__ void get_chunk(const float *s, float2 (&c)[2][2]) {
+    const float4 u = reinterpret_cast<const float4 *>(s)[0], v = reinterpret_cast<const float4 *>(s)[1];
+    c[0][0] = lo2(u);
+    c[0][1] = hi2(u);
+    c[1][0] = lo2(v);
+    c[1][1] = hi2(v);
+}
+
+// Shared memory of a CTA: the sweeps' publications, the chunks sent, the chunks received and,
+// for every message received, where it comes from.
+template <int NW, int R>
+struct ResSmem {
+    static constexpr int chunks = res_chunks(NW * R), msgs = res_msgs(NW * R);
+    static constexpr int out = 2 * NW * 128 * 16;        // bytes
+    static constexpr int in = out + chunks * 32 + 16;    // (a chunk's third message reads 1 float past it)
+    static constexpr int src = in + chunks * 32 + 16;
+    static constexpr int bytes = src + msgs * 4;
+};
+
+// A CTA's tile of its image, seen from one lane.
+struct ResTile {
+    int tile, tx, ty, ntx, nty;
+    int H, W, ld;
+    int y0, y1;            // its own rows
+    int own;               // lanes 1 .. own hold its own columns
+    int xa;                // the lane's first column (a multiple of 4)
+    bool nl, nr, nu, nd;   // neighbours
+    bool own_col, col_in;  // the lane's columns are the tile's own / start inside the image
+    int side;              // res_neighbours' SIDE
+    bool ghosts;           // the warp holds a ghost row
+};
+
+template <int R>
+__device__ __forceinline__ void res_tile(ResTile &g, ResLane &t, int tile, int ntx, int nty, int H, int W, int ld,
+                                         unsigned tmem) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    g.tile = tile;
+    g.ntx = ntx;
+    g.nty = nty;
+    g.tx = tile % ntx;
+    g.ty = tile / ntx;
+    g.H = H;
+    g.W = W;
+    g.ld = ld;
+    const int chunks = (W + 3) / 4;
+    const int x0 = 4 * res_split(g.tx, ntx, chunks), x1 = 4 * res_split(g.tx + 1, ntx, chunks);
+    g.y0 = res_split(g.ty, nty, H);
+    g.y1 = res_split(g.ty + 1, nty, H);
+    g.own = (x1 - x0) / 4;
+    g.xa = x0 - 4 + 4 * lane;
+    g.nl = g.tx > 0;
+    g.nr = g.tx + 1 < ntx;
+    g.nu = g.ty > 0;
+    g.nd = g.ty + 1 < nty;
+    // every plane row holds whole chunks (ld % 4 == 0), so a chunk that starts inside the image
+    // may be read; other chunks are never needed
+    g.col_in = g.xa >= 0 && g.xa < W;
+    g.own_col = lane >= 1 && lane <= g.own;
+    g.side = g.nl && g.nr ? -1 : (W - 1) & 3;
+    t.lane = lane;
+    t.warp = warp;
+    t.first = g.xa == 0;
+    t.last = g.xa <= W - 1 && g.xa + 4 > W - 1;
+    t.row0 = g.y0 - kResT + warp * R;
+    t.H = H;
+    t.tmem = tmem + ((unsigned)(warp & 3) << 21) + (unsigned)(warp >> 2) * (R * 16);
+    g.ghosts = (t.row0 < 0 && t.row0 + R > 0) || (t.row0 < H && t.row0 + R > H);
+}
+
+// Where each message a tile receives comes from: its index in all outboxes' first half, -1: none;
+// and the chunks nobody sends stay 0 (cells that are never used, but garbage there, a NaN, would
+// send whole warps through the exact form's general division).
+template <int NW, int R>
+__device__ __forceinline__ void res_sources(const ResTile &g, int *src, float *in) {
+    using S = ResSmem<NW, R>;
+    const int chunks = (g.W + 3) / 4;
+    const int lown = g.nl ? res_split(g.tx, g.ntx, chunks) - res_split(g.tx - 1, g.ntx, chunks) : 0;
+    for (int i = threadIdx.x; i < S::msgs; i += NW * 32) {
+        const int c = i / 3, m = i % 3;
+        int dx = 0, dy = 0, from = -1;  // the neighbour and its chunk
+        if (c < 2 * kResRowChunks) {
+            const int blk = c / kResRowChunks, l = c % 32;  // 0: above, from that tile's last rows
+            dy = blk == 0 ? -1 : 1;
+            dx = l == 0 ? -1 : l == g.own + 1 ? 1 : 0;
+            if (l <= g.own + 1)
+                from = (1 - blk) * kResRowChunks + (c % kResRowChunks) - l + (l == 0 ? lown : l == g.own + 1 ? 1 : l);
+        } else {
+            const int k = c - 2 * kResRowChunks, sd = k >= NW * R, lr = k - sd * (NW * R);
+            dx = sd ? 1 : -1;
+            const int row = g.y0 - kResT + lr;
+            if (row >= g.y0 && row < g.y1) from = 2 * kResRowChunks + (1 - sd) * (NW * R) + lr;
+        }
+        const int nx = g.tx + dx, ny = g.ty + dy;
+        if (nx < 0 || nx >= g.ntx || ny < 0 || ny >= g.nty) from = -1;
+        src[i] = from < 0 ? -1 : (ny * g.ntx + nx) * S::msgs + 3 * from + m;
+    }
+    for (int i = threadIdx.x; i < S::chunks * 8; i += NW * 32) in[i] = 0.f;
+}
+
+// Exchange e of a tile (all threads of the CTA): the ring of cu to the neighbours, their rings into
+// its halo.  FENCE: what this CTA wrote to global memory before the exchange is visible to its
+// neighbours after it.  false: a wait ran out.
+template <int NW, int R, bool FENCE>
+__device__ __forceinline__ bool res_exchange(const ResLane &t, const ResTile &g, float2 (&cu)[R][2][2], float *out,
+                                             float *in, const int *src, float4 *box, unsigned e, int *stop,
+                                             unsigned *abort_flag, int *status) {
+    using S = ResSmem<NW, R>;
+    // (uniform in the warp) rows of the ring, and rows of the halo, among the warp's
+    const int row_end = t.row0 + R;
+    const bool up_rows = t.row0 < g.y0 + kResT && row_end > g.y0;
+    const bool down_rows = t.row0 < g.y1 && row_end > g.y1 - kResT;
+    const bool above_rows = t.row0 < g.y0, below_rows = t.row0 < g.y1 + kResT && row_end > g.y1;
+    if constexpr (FENCE) __threadfence();
+    if ((t.lane == 1 && g.nl) || (t.lane == g.own && g.nr)) {  // (own >= 2 in a tile with neighbours beside it)
+        float *f = out + 8 * (2 * kResRowChunks + (t.lane == 1 ? 0 : NW * R) + t.warp * R);
+#pragma unroll
+        for (int r = 0; r < R; ++r) put_chunk(f + 8 * r, cu[r]);
+    }
+    if (up_rows || down_rows) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int j = t.row0 + r - g.y0, k = t.row0 + r - (g.y1 - kResT);
+            if (j >= 0 && j < kResT) put_chunk(out + 8 * (32 * j + t.lane), cu[r]);
+            if (k >= 0 && k < kResT) put_chunk(out + 8 * (kResRowChunks + 32 * k + t.lane), cu[r]);
+        }
+    }
+    __syncthreads();
+    float4 *boxes = box + ((e & 1u) ? (size_t)g.ntx * g.nty * S::msgs : 0);
+    float4 *mine = boxes + (size_t)g.tile * S::msgs;
+    constexpr int kPer = (S::msgs + NW * 32 - 1) / (NW * 32);  // messages per thread
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const int m = threadIdx.x + i * NW * 32;
+        if (m < S::msgs) {
+            const float *f = out + 8 * (m / 3) + 3 * (m % 3);
+            msg_store(mine + m, f[0], f[1], f[2], e);
+        }
+    }
+    // receive: all of the thread's loads in flight, until each carries e
+    int from[kPer];
+    float got[kPer][3];
+    unsigned tag[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const int m = threadIdx.x + i * NW * 32;
+        from[i] = m < S::msgs ? src[m] : -1;
+        tag[i] = e;
+        if (from[i] >= 0) msg_load(boxes + from[i], got[i], tag[i]);
+    }
+    for (int polls = 0;;) {
+        bool all = true;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) all = all && tag[i] == e;
+        if (all) break;
+        if (++polls > kResPolls ||
+            ((polls & 1023) == 0 && (*(volatile int *)stop || *(volatile unsigned *)abort_flag))) {
+            atomicExch(abort_flag, 1u);
+            if (status) atomicCAS(status, 0, (int)HS_ERR_TIMEOUT);
+            *(volatile int *)stop = 1;
+            break;
+        }
+#pragma unroll
+        for (int i = 0; i < kPer; ++i)
+            if (tag[i] != e) msg_load(boxes + from[i], got[i], tag[i]);
+    }
+    if constexpr (FENCE) __threadfence();
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const int m = threadIdx.x + i * NW * 32;
+        if (from[i] >= 0) {
+            float *f = in + 8 * (m / 3) + 3 * (m % 3);
+            f[0] = got[i][0];
+            f[1] = got[i][1];
+            if (m % 3 < 2) f[2] = got[i][2];
+        }
+    }
+    __syncthreads();
+    if (*(volatile int *)stop) return false;
+    if ((t.lane == 0 && g.nl) || (t.lane == g.own + 1 && g.nr)) {
+        const float *f = in + 8 * (2 * kResRowChunks + (t.lane == 0 ? 0 : NW * R) + t.warp * R);
+#pragma unroll
+        for (int r = 0; r < R; ++r) get_chunk(f + 8 * r, cu[r]);
+    }
+    if ((above_rows && g.nu) || (below_rows && g.nd)) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int j = t.row0 + r - (g.y0 - kResT), k = t.row0 + r - g.y1;
+            if (g.nu && j < kResT) get_chunk(in + 8 * (32 * j + t.lane), cu[r]);
+            if (g.nd && k >= 0 && k < kResT) get_chunk(in + 8 * (kResRowChunks + 32 * k + t.lane), cu[r]);
+        }
+    }
+    __syncwarp();
+    return true;
+}
+
+// n sweeps in the variant of the tile's side (uniform in the CTA; one block barrier per sweep).
+template <bool FAST, int NW, int R, bool UPDATE = true>
+__device__ __forceinline__ void res_run(const ResLane &t, const ResTile &g, float2 (&cu)[R][2][2], float4 *pub,
+                                        int half, int n, float we, float wc) {
+    switch (g.side) {
+        case -1: res_sweeps<FAST, NW, R, -1, UPDATE>(t, cu, pub, half, n, g.ghosts, we, wc); break;
+        case 0: res_sweeps<FAST, NW, R, 0, UPDATE>(t, cu, pub, half, n, g.ghosts, we, wc); break;
+        case 1: res_sweeps<FAST, NW, R, 1, UPDATE>(t, cu, pub, half, n, g.ghosts, we, wc); break;
+        case 2: res_sweeps<FAST, NW, R, 2, UPDATE>(t, cu, pub, half, n, g.ghosts, we, wc); break;
+        default: res_sweeps<FAST, NW, R, 3, UPDATE>(t, cu, pub, half, n, g.ghosts, we, wc); break;
+    }
+}
+
+// The tile's own pixels of the state to planes U, V.
+template <int R>
+__device__ __forceinline__ void res_store_own(const ResLane &t, const ResTile &g, const float2 (&cu)[R][2][2],
+                                              float *U, float *V) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int row = t.row0 + r;
+        if (row >= g.y0 && row < g.y1 && g.own_col) res_store(U, V, (size_t)row * g.ld + g.xa, g.W - g.xa, cu[r]);
+    }
+    __syncwarp();
 }
 
 }  // namespace hs

@@ -32,6 +32,8 @@
 // and multiplies by a reciprocal of the denominator computed once per row per pass.
 #pragma once
 
+#include <vector>
+
 #include "hs_common.cuh"
 
 namespace hs {
@@ -452,6 +454,28 @@ struct ResidentJob {
 };
 hs_status run_resident_jobs(const ResidentJob *jobs, int n, int ckpt_every, size_t ckpt_plane, int *status,
                             const ResolvedConfig &rc, cudaStream_t s);
+// The backward of run_resident_jobs' training form (hs_resident_adj.cu): the accumulators dIx, dIy,
+// dIt and the tiles' shares of dL/dalpha^2 (nslots per image).  HS_ERR_UNSUPPORTED as there, or when
+// the streaming passes are the faster ones.
+struct ResidentAdjJob {
+    const float *Ix, *Iy, *It, *dLdu, *dLdv, *ckpt;
+    float *states, *park, *acc;
+    double *a2part;
+    char *scratch;
+    size_t scratch_bytes;
+    const float *alpha_dev;
+    int H, W, ld;
+};
+hs_status run_resident_adjoint(const ResidentAdjJob *jobs, int n, int iters, int ckpt_every, size_t plane, int nslots,
+                               const ResolvedConfig &rc, cudaStream_t s);
+// How jobs, in their order, are cut into launches: launch k holds jobs end[k-1] .. end[k]-1 with
+// r[k] <= max_r rows per warp; a sweep of a launch takes base + slope * r us.
+struct ResidentCut {
+    std::vector<int> end, r;
+};
+bool resident_cut(const ResidentJob *jobs, int n, double base, double slope, int max_r, ResidentCut &cut);
+int resident_tiles(int H, int W, int r, int *ntx, int *nty);
+size_t resident_box_bytes(int tiles, int r);
 // A depth, a segment size or a layout in hs_config asks for the streaming passes.
 inline bool wants_resident(const ResolvedConfig &rc) { return rc.T_default && rc.seg_rows == 0 && rc.layout == 0; }
 inline size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }

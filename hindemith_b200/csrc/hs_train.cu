@@ -792,6 +792,35 @@ static hs_status side_stream(int dev, SideStream **out) {
     return HS_OK;
 }
 
+// The end of the backward: transposed derivative stencils and dalpha.
+static hs_status train_finish(const hs_train_pair *pairs, const PairBufs *bufs, int n, int nslots, cudaStream_t s) {
+    FinishTable ft;
+    memset(&ft, 0, sizeof(ft));
+    ft.npairs = n;
+    int maxW = 1, maxH = 1;
+    for (int i = 0; i < n; ++i) {
+        const PairBufs &B = bufs[i];
+        ft.dIx[i] = B.accum(0);
+        ft.dIy[i] = B.accum(1);
+        ft.dIt[i] = B.accum(2);
+        ft.a2part[i] = B.a2part;
+        ft.dI0[i] = pairs[i].dI0;
+        ft.dI1[i] = pairs[i].dI1;
+        ft.alpha[i] = pairs[i].alpha;
+        ft.dalpha[i] = pairs[i].dalpha;
+        ft.H[i] = pairs[i].H;
+        ft.W[i] = pairs[i].W;
+        ft.ld[i] = pairs[i].ld;
+        maxW = std::max(maxW, pairs[i].W);
+        maxH = std::max(maxH, pairs[i].H);
+    }
+    batch_derivs_adjoint_kernel<<<dim3((maxW + 63) / 64, (maxH + 3) / 4, n), dim3(64, 4), 0, s>>>(ft);
+    HS_LAUNCH_CHECK("batch_derivs_adjoint_kernel");
+    batch_fold_kernel<<<n, 256, 0, s>>>(ft, nslots);
+    HS_LAUNCH_CHECK("batch_fold_kernel");
+    return HS_OK;
+}
+
 // Backward of train_forward (the same buffers): per checkpoint interval in reverse, dump
 // passes recompute the interval's states, then adjoint passes of balanced depth reverse its
 // sweeps; last the transposed derivative stencils and the dalpha fold.
@@ -806,6 +835,22 @@ static hs_status train_backward(const hs_train_pair *pairs, const PairBufs *bufs
                                 int ckpt_every, int nslots, const ResolvedConfig &rc,
                                 cudaStream_t s) {
     hs_status st;
+    // Images that fit the chip are reversed there (hs_resident_adj.cu).  The exchange scratch is
+    // the forward's ping-pong buffers, or lambda's second buffer in the single-pair call.
+    if (wants_resident(rc)) {
+        std::vector<ResidentAdjJob> jobs(n);
+        for (int i = 0; i < n; ++i) {
+            const hs_train_pair &d = pairs[i];
+            const PairBufs &B = bufs[i];
+            jobs[i] = {B.deriv(0), B.deriv(1), B.deriv(2), d.dLdu, d.dLdv, B.ck(0, 0),
+                       reinterpret_cast<float *>(B.states), B.lamb(0, 0), B.accum(0), B.a2part,
+                       B.scratch ? B.scratch : reinterpret_cast<char *>(B.lamb(1, 0)),
+                       (B.scratch ? 4 : 2) * B.pb, d.alpha, d.H, d.W, d.ld};
+        }
+        st = run_resident_adjoint(jobs.data(), n, iters, ckpt_every, bufs[0].pb / sizeof(float), nslots, rc, s);
+        if (st == HS_OK) return train_finish(pairs, bufs, n, nslots, s);
+        if (st != HS_ERR_UNSUPPORTED) return st;
+    }
     for (int i = 0; i < n; ++i) {
         const PairBufs &B = bufs[i];
         const size_t pl = plane_bytes(pairs[i].H, pairs[i].ld);
@@ -972,32 +1017,7 @@ static hs_status train_backward(const hs_train_pair *pairs, const PairBufs *bufs
         jhi -= tb;
     }
 
-    // 3. transposed derivative stencils and dalpha
-    FinishTable ft;
-    memset(&ft, 0, sizeof(ft));
-    ft.npairs = n;
-    int maxW = 1, maxH = 1;
-    for (int i = 0; i < n; ++i) {
-        const PairBufs &B = bufs[i];
-        ft.dIx[i] = B.accum(0);
-        ft.dIy[i] = B.accum(1);
-        ft.dIt[i] = B.accum(2);
-        ft.a2part[i] = B.a2part;
-        ft.dI0[i] = pairs[i].dI0;
-        ft.dI1[i] = pairs[i].dI1;
-        ft.alpha[i] = pairs[i].alpha;
-        ft.dalpha[i] = pairs[i].dalpha;
-        ft.H[i] = pairs[i].H;
-        ft.W[i] = pairs[i].W;
-        ft.ld[i] = pairs[i].ld;
-        maxW = std::max(maxW, pairs[i].W);
-        maxH = std::max(maxH, pairs[i].H);
-    }
-    batch_derivs_adjoint_kernel<<<dim3((maxW + 63) / 64, (maxH + 3) / 4, n), dim3(64, 4), 0, s>>>(ft);
-    HS_LAUNCH_CHECK("batch_derivs_adjoint_kernel");
-    batch_fold_kernel<<<n, 256, 0, s>>>(ft, nslots);
-    HS_LAUNCH_CHECK("batch_fold_kernel");
-    return HS_OK;
+    return train_finish(pairs, bufs, n, nslots, s);
 }
 
 static size_t plane_stride(int H, int ld) { return round_up(plane_bytes(H, ld), 256); }

@@ -160,9 +160,10 @@ def _log(entry):
 
 def best_batch_config(specs, fast_math: bool = True, candidates=BATCH_CANDIDATES,
                       reps: int = 3) -> Tuple[int, int, int]:
-    """(sweeps_per_pass, rows_per_segment, layout) fastest for the persistent batched launch of
-    `specs` = [(H, W, alpha, iters)] on the current device (timed as CUDA-graph replays
-    of the batch itself over seeded random planes)."""
+    """(sweeps_per_pass, rows_per_segment, layout) fastest for the batched call of `specs` =
+    [(H, W, alpha, iters)] on the current device (timed as CUDA-graph replays of the batch
+    itself over seeded random planes): the persistent launch under each candidate, and
+    (0, 0, 0), the library's own choice."""
     import hashlib
 
     import torch
@@ -181,8 +182,8 @@ def best_batch_config(specs, fast_math: bool = True, candidates=BATCH_CANDIDATES
     g = torch.Generator(device="cuda")
     g.manual_seed(0)
     results = []
-    for T, rows, layout in candidates:
-        if layout != 1 and not fast_math:
+    for T, rows, layout in (*candidates, (0, 0, 0)):
+        if layout == 2 and not fast_math:
             if (T, rows, 1) in candidates:
                 continue
             layout = 1

@@ -158,9 +158,11 @@ typedef struct hs_pair_desc {
 HS_API size_t hs_forward_batched_workspace_bytes(const hs_pair_desc *pairs, int n,
                                                  const hs_config *cfg);
 
-/* hs_forward for n (1..HS_MAX_BATCH) pairs of uneven size in one persistent launch:
- * every (pass, pair, tile) is a work item taken from a device queue; a tile waits only
- * for its neighbours' previous pass (bounded waits).  Results equal hs_forward per pair.
+/* hs_forward for n (1..HS_MAX_BATCH) pairs of uneven size.  With sweeps_per_pass,
+ * rows_per_segment and layout all 0 the pairs that fit the chip run there, as many at a time as
+ * the SMs hold, each larger one in its own passes; otherwise one persistent launch: every (pass,
+ * pair, tile) is a work item taken from a device queue; a tile waits only for its neighbours'
+ * previous pass.  All waits are bounded.  Results equal hs_forward per pair.
  * Stream-ordered and free of host synchronisation, allocation and pageable copies, so it
  * can be captured in a CUDA graph (make one call before capturing: the first call sets
  * kernel attributes).  `device_status` (device int, may be NULL) receives HS_OK or
@@ -223,7 +225,9 @@ typedef struct hs_train_pair {
 HS_API size_t hs_train_workspace_bytes(const hs_train_pair *pairs, int n, int iters, int ckpt_every);
 
 /* Forward of n pairs with checkpoints every ckpt_every sweeps kept in the workspace; each
- * pass is one launch over all pairs.  Results equal hs_forward per pair. */
+ * pass is one launch over all pairs, or, when the pairs fit the chip and no depth, segment or
+ * layout is given, all sweeps of a group of pairs are one launch.  Results equal hs_forward per
+ * pair. */
 HS_API hs_status hs_forward_train_batched(const hs_train_pair *pairs, int n, int iters,
                                           int ckpt_every, void *workspace, size_t workspace_bytes,
                                           const hs_config *cfg, void *stream);
@@ -234,7 +238,9 @@ HS_API hs_status hs_forward_train_batched(const hs_train_pair *pairs, int n, int
  * ahead, and the adjoint runs temporally blocked on the caller's stream, min(4,
  * sweeps_per_pass) adjoint sweeps per HBM pass in passes of balanced depth that may span
  * two intervals.  The side stream joins a capture of the caller's stream through events and
- * is joined back before the call returns.  Needs alpha != 0.  Deterministic. */
+ * is joined back before the call returns.  Small groups of pairs that fit the chip are reversed
+ * there in one launch when no depth, segment or layout is given.  Needs alpha != 0.
+ * Deterministic. */
 HS_API hs_status hs_backward_batched(const hs_train_pair *pairs, int n, int iters, int ckpt_every,
                                      void *workspace, size_t workspace_bytes,
                                      const hs_config *cfg, void *stream);

@@ -422,8 +422,8 @@ hs_status hs_forward_batched(const hs_pair_desc *pairs, int n, void *workspace,
     // longest first, as many at a time as the SMs hold, and each larger one in its own passes.  The
     // persistent kernel below serves explicit settings: its chains of dependent passes leave the
     // chip idle unless many tiles are independent (measured on B200, fast form, Gpix-it/s, at its
-    // default depth 4 -> this way: 16 mixed pairs 500 -> 660, 3 of 2048^2 423 -> 690, 8 of 640x480
-    // 183 -> 420).
+    // default depth 4 -> this way: 16 mixed pairs 545 -> 672, 3 of 2048^2 528 -> 649, 8 of 640x480
+    // 185 -> 628, 12 of 320x240 84 -> 474).
     if (wants_resident(rc)) {
         if (device_status) HS_CUDA_CHECK(cudaMemsetAsync(device_status, 0, sizeof(int), s));
         std::vector<int> in;

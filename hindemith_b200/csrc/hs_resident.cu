@@ -3,8 +3,8 @@
 //
 // Measured on one B200 (hs_forward, us per call, streaming passes at their default depth ->
 // resident):
-//   1920x1080 x 500 sweeps, fast   2001 -> 1207      1901x1037 x 200, exact  1463 -> 970
-//   320x240 x 100, fast             171 ->  107       640x480 x 200, exact    856 -> 310
+//   1920x1080 x 500 sweeps, fast   2003 -> 1244      1901x1037 x 200, exact  1464 -> 958
+//   320x240 x 100, fast             171 ->  112       640x480 x 200, exact    855 -> 317
 // Bound (1080p, fast, 16 x 8 rows): of 2.4 us per sweep, 1.7 us are the sweep itself (the FP32
 // pipe and the register reads of its packed operations: fma.rn.f32x2 with three distinct
 // operands issues every 3.1 clocks, with a shared one every 2.2) and 0.7 us the exchange's share

@@ -424,7 +424,7 @@ hs_status hs_forward_batched(const hs_pair_desc *pairs, int n, void *workspace,
     // chip idle unless many tiles are independent (measured on B200, fast form, Gpix-it/s, at its
     // default depth 4 -> this way: 16 mixed pairs 545 -> 672, 3 of 2048^2 528 -> 649, 8 of 640x480
     // 185 -> 628, 12 of 320x240 84 -> 474).
-    if (wants_resident(rc)) {
+    if (wants_resident(rc) && outputs_apart(pairs, n)) {
         if (device_status) HS_CUDA_CHECK(cudaMemsetAsync(device_status, 0, sizeof(int), s));
         std::vector<int> in;
         for (int i = 0; i < n; ++i)

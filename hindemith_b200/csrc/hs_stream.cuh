@@ -32,6 +32,7 @@
 // and multiplies by a reciprocal of the denominator computed once per row per pass.
 #pragma once
 
+#include <algorithm>
 #include <vector>
 
 #include "hs_common.cuh"
@@ -476,6 +477,40 @@ struct ResidentCut {
 bool resident_cut(const ResidentJob *jobs, int n, double base, double slope, int max_r, ResidentCut &cut);
 int resident_tiles(int H, int W, int r, int *ntx, int *nty);
 size_t resident_box_bytes(int tiles, int r);
+// Whether the outputs u, v of n pairs lie apart from the images I0, I1 of all of them, or take the
+// place of one of their own pair's images exactly.  The passes read every image before they write
+// any output; in the resident form a tile reads its own pixels and its neighbours' before any of
+// these is written, and no more: an output that shares memory with an image in any other way (at
+// an offset, or with another pair's image) takes the passes.
+template <class Pair>
+bool outputs_apart(const Pair *pairs, int n) {
+    struct Range {
+        uintptr_t lo, hi;
+        int pair;
+    };
+    std::vector<Range> im;
+    im.reserve(2 * n);
+    auto range = [&](const float *p, int i) {
+        const uintptr_t lo = reinterpret_cast<uintptr_t>(p);
+        return Range{lo, lo + plane_bytes(pairs[i].H, pairs[i].ld), i};
+    };
+    for (int i = 0; i < n; ++i) {
+        im.push_back(range(pairs[i].I0, i));
+        im.push_back(range(pairs[i].I1, i));
+    }
+    std::sort(im.begin(), im.end(), [](const Range &a, const Range &b) { return a.lo < b.lo; });
+    std::vector<uintptr_t> reach(2 * n);  // the furthest end of im[0 .. k]
+    for (int k = 0; k < 2 * n; ++k) reach[k] = std::max(im[k].hi, k ? reach[k - 1] : 0);
+    for (int i = 0; i < 2 * n; ++i) {
+        const Range o = range(i & 1 ? pairs[i / 2].v : pairs[i / 2].u, i / 2);
+        int k = (int)(std::lower_bound(im.begin(), im.end(), o.hi,
+                                   [](const Range &a, uintptr_t x) { return a.lo < x; }) - im.begin());
+        if (k == 0 || reach[k - 1] <= o.lo) continue;
+        while (--k >= 0)
+            if (im[k].hi > o.lo && !(im[k].pair == o.pair && im[k].lo == o.lo)) return false;
+    }
+    return true;
+}
 // A depth, a segment size or a layout in hs_config asks for the streaming passes.
 inline bool wants_resident(const ResolvedConfig &rc) { return rc.T_default && rc.seg_rows == 0 && rc.layout == 0; }
 inline size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }

@@ -407,8 +407,12 @@ hs_status hs_forward(const float *I0, const float *I1, int H, int W, int ld, flo
     float *u1 = reinterpret_cast<float *>(w + 3 * pb);
     float *v1 = reinterpret_cast<float *>(w + 4 * pb);
     cudaStream_t s = (cudaStream_t)stream;
+    hs_pair_desc self = {};
+    self.I0 = I0; self.I1 = I1;
+    self.u = u; self.v = v;
+    self.H = H; self.ld = ld;
     ResidentPlan pl;
-    if (wants_resident(rc) && resident_plan(H, W, iters, need, pl)) {
+    if (wants_resident(rc) && resident_plan(H, W, iters, need, pl) && outputs_apart(&self, 1)) {
         st = run_resident(I0, I1, nullptr, nullptr, nullptr, H, W, ld, alpha * alpha, iters, u, v, workspace, true,
                           rc, pl, s);
         if (st != HS_ERR_UNSUPPORTED) return st;

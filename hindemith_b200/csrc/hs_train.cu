@@ -715,7 +715,7 @@ static hs_status train_forward(const hs_train_pair *pairs, const PairBufs *bufs,
     // Images that fit the chip run there for all sweeps (hs_resident.cuh), in groups of as many
     // as fit at once: one launch instead of one per pass, and no state traffic but the
     // checkpoints.  The exchange scratch is the passes' ping-pong buffers.
-    if (wants_resident(rc)) {
+    if (wants_resident(rc) && outputs_apart(pairs, n)) {
         std::vector<ResidentJob> jobs(n);
         for (int i = 0; i < n; ++i) {
             const hs_train_pair &d = pairs[i];

@@ -1,0 +1,111 @@
+"""Which kernels a call takes, on a CPU: the library's host code on a recording CUDA runtime
+(fake_cuda).  Pointers are only numbers here."""
+import ctypes
+
+import pytest
+
+from fake_cuda import fake_cuda
+from hindemith_b200 import _lib as L
+
+P = ctypes.c_void_p
+MB = 1 << 20
+WS = 1 << 40  # a workspace far from all planes
+
+
+@pytest.fixture()
+def fake():
+    return fake_cuda()
+
+
+def pad(W):
+    return (W + 3) // 4 * 4
+
+
+def forward(fake, H, W, iters, I0, I1, u, v, cfg=None):
+    cfg = cfg if cfg is not None else L.make_config(fast_math=True)
+    ld = pad(W)
+    need = fake.lib.hs_forward_workspace_bytes(H, W, ld)
+    assert fake.lib.hs_forward(P(I0), P(I1), H, W, ld, 1.0, iters, P(u), P(v), P(WS), need, ctypes.byref(cfg), None) == L.HS_OK
+    return fake.launches()
+
+
+def batch(fake, specs, cfg=None, planes=None):
+    """hs_forward_batched of (H, W, iters) pairs; planes[i] = (I0, I1, u, v), else all apart."""
+    cfg = cfg if cfg is not None else L.make_config(fast_math=True)
+    arr = (L.hs_pair_desc * len(specs))()
+    for i, (d, (H, W, iters)) in enumerate(zip(arr, specs)):
+        at = planes[i] if planes else [(1 << 36) + (4 * i + k) * 64 * MB for k in range(4)]
+        d.I0, d.I1, d.u, d.v = at
+        d.H, d.W, d.ld, d.alpha, d.iters = H, W, pad(W), 1.0, iters
+    need = fake.lib.hs_forward_batched_workspace_bytes(arr, len(specs), ctypes.byref(cfg))
+    assert need > 0
+    assert fake.lib.hs_forward_batched(arr, len(specs), P(WS), need, ctypes.byref(cfg), None, None) == L.HS_OK
+    return fake.launches()
+
+
+def train_pairs(shapes, planes=None):
+    arr = (L.hs_train_pair * len(shapes))()
+    for i, (d, (H, W)) in enumerate(zip(arr, shapes)):
+        at = planes[i] if planes else [(1 << 36) + (8 * i + k) * 64 * MB for k in range(4)]
+        d.I0, d.I1, d.u, d.v = at
+        base = (1 << 37) + 8 * i * 64 * MB
+        d.dLdu, d.dLdv, d.dI0, d.dI1 = (base + k * 64 * MB for k in range(4))
+        d.alpha, d.dalpha = 1 << 35, (1 << 35) + 256 + 4 * i
+        d.H, d.W, d.ld = H, W, pad(W)
+    return arr
+
+
+def train(fake, shapes, iters, ckpt, cfg=None, planes=None, backward=False):
+    cfg = cfg if cfg is not None else L.make_config(fast_math=True)
+    arr = train_pairs(shapes, planes)
+    need = fake.lib.hs_train_workspace_bytes(arr, len(shapes), iters, ckpt)
+    call = fake.lib.hs_backward_batched if backward else fake.lib.hs_forward_train_batched
+    assert call(arr, len(shapes), iters, ckpt, P(WS), need, ctypes.byref(cfg), None) == L.HS_OK
+    return fake.launches()
+
+
+def kernels(launches):
+    return {x.kernel for x in launches}
+
+
+# ------------------------------------------------------------------ outputs over images
+
+A, B, C, D = ((k + 1) << 32 for k in range(4))
+
+
+@pytest.mark.parametrize("u,v,resident", [(C, D, True), (A, B, True), (B, A, True), (A, C, True),
+                                          (A + 1280, C, False), (C, B - 1280, False), (A - 480 * 640 * 4, B + 480 * 640 * 4, True),
+                                          (A - 480 * 640 * 4 + 16, C, False)])
+def test_forward_with_an_output_inside_an_image(fake, u, v, resident):
+    """In the place of an image, or apart: on the chip.  At an offset: the passes, which have read
+    all of the images before they write."""
+    ks = kernels(forward(fake, 480, 640, 20, A, B, u, v))
+    assert ("hs_resident_kernel" in ks) == resident
+    assert ("derivs_kernel" in ks) == (not resident)
+
+
+def test_batch_with_an_output_over_another_pairs_image(fake):
+    """Frames of a sequence, the flow of pair 0 over a frame that pair 1 reads: no pair may write
+    before all have read."""
+    H, W = 240, 320
+    frames = [(1 << 36) + k * 64 * MB for k in range(3)]
+    out = [(1 << 37) + k * 64 * MB for k in range(4)]
+    pairs = [(frames[0], frames[1], out[0], frames[1]), (frames[1], frames[2], out[2], out[3])]
+    apart = [(frames[0], frames[1], out[0], out[1]), (frames[1], frames[2], out[2], out[3])]
+    own = [(frames[0], frames[1], frames[0], out[1]), (frames[1], frames[2], out[2], frames[2])]
+    assert "batch_derivs_kernel" in kernels(batch(fake, [(H, W, 20)] * 2, planes=pairs))
+    for ok in (apart, own):
+        fake.reset()
+        assert kernels(batch(fake, [(H, W, 20)] * 2, planes=ok)) == {"res_clear_kernel", "hs_resident_kernel"}
+
+
+def test_training_forward_with_an_output_over_another_pairs_image(fake):
+    H, W = 240, 320
+    frames = [(1 << 36) + k * 64 * MB for k in range(3)]
+    out = [(1 << 38) + k * 64 * MB for k in range(4)]
+    pairs = [(frames[0], frames[1], out[0], frames[2]), (frames[1], frames[2], out[2], out[3])]
+    apart = [(frames[0], frames[1], out[0], out[1]), (frames[1], frames[2], out[2], out[3])]
+    ks = kernels(train(fake, [(H, W)] * 2, 20, 5, planes=pairs))
+    assert "derivs_kernel" in ks and "hs_resident_kernel" not in ks
+    fake.reset()
+    assert "hs_resident_kernel" in kernels(train(fake, [(H, W)] * 2, 20, 5, planes=apart))

@@ -446,11 +446,11 @@ hs_status hs_forward_batched(const hs_pair_desc *pairs, int n, void *workspace,
             j.H = d.H; j.W = d.W; j.ld = d.ld;
             j.iters = d.iters;
         }
-        st = jobs.empty() ? HS_OK : run_resident_jobs(jobs.data(), (int)jobs.size(), 0, 0, device_status, rc, s);
+        int launched = 0;
+        st = run_resident_jobs(jobs.data(), (int)jobs.size(), 0, 0, device_status, rc, s, &launched);
         if (st != HS_OK && st != HS_ERR_UNSUPPORTED) return st;
         std::vector<char> done(n, 0);
-        if (st == HS_OK)
-            for (int i : in) done[i] = 1;
+        for (int k = 0; k < launched; ++k) done[in[k]] = 1;
         for (int i = 0; i < n; ++i) {
             const hs_pair_desc &d = pairs[i];
             if (done[i]) continue;

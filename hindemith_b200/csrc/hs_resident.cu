@@ -334,7 +334,8 @@ bool resident_fits(int H, int W, int iters, size_t scratch_bytes) {
 }
 
 hs_status run_resident_jobs(const ResidentJob *jobs, int n, int ckpt_every, size_t ckpt_plane, int *status,
-                            const ResolvedConfig &rc, cudaStream_t s) {
+                            const ResolvedConfig &rc, cudaStream_t s, int *launched) {
+    *launched = 0;
     for (int i = 0; i < n; ++i)
         if (jobs[i].iters < 2) return HS_ERR_UNSUPPORTED;
     ResidentCut cut;
@@ -366,6 +367,7 @@ hs_status run_resident_jobs(const ResidentJob *jobs, int n, int ckpt_every, size
         }
         const hs_status st = launch_table(tab, r, true, rc, s);
         if (st != HS_OK) return st;
+        *launched = i0 + m;
     }
     return HS_OK;
 }

@@ -443,7 +443,10 @@ bool resident_fits(int H, int W, int iters, size_t scratch_bytes);
 // many as fit the chip at once; the flow goes to u, v.  Training: derivatives into Ix, Iy, It (may
 // be null), the state after every ckpt_every sweeps into the checkpoint planes (ckpt_plane floats
 // apart; u then v).  status, if set, receives HS_ERR_TIMEOUT when a wait runs out.
-// HS_ERR_UNSUPPORTED when an image does not fit (any launches made are to be redone).
+// *launched: the jobs, the first so many, whose launches were made.  HS_ERR_UNSUPPORTED when an
+// image does not fit, or the SMs at hand hold fewer tiles than the device: the caller runs the
+// jobs that were not launched in another way, and those only (a flow may have taken the place of
+// its own image).
 struct ResidentJob {
     const float *I0, *I1;
     float *Ix, *Iy, *It, *u, *v, *ckpt;
@@ -454,7 +457,7 @@ struct ResidentJob {
     int H, W, ld, iters;
 };
 hs_status run_resident_jobs(const ResidentJob *jobs, int n, int ckpt_every, size_t ckpt_plane, int *status,
-                            const ResolvedConfig &rc, cudaStream_t s);
+                            const ResolvedConfig &rc, cudaStream_t s, int *launched);
 // The backward of run_resident_jobs' training form (hs_resident_adj.cu): the accumulators dIx, dIy,
 // dIt and the tiles' shares of dL/dalpha^2 (nslots per image).  HS_ERR_UNSUPPORTED as there, or when
 // the streaming passes are the faster ones.

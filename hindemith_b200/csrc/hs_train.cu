@@ -723,8 +723,12 @@ static hs_status train_forward(const hs_train_pair *pairs, const PairBufs *bufs,
             jobs[i] = {d.I0, d.I1, B.deriv(0), B.deriv(1), B.deriv(2), d.u, d.v, B.ck(0, 0), B.scratch,
                        4 * B.pb, d.alpha, 0.f, d.H, d.W, d.ld, iters};
         }
-        st = run_resident_jobs(jobs.data(), n, ckpt_every, bufs[0].pb / sizeof(float), nullptr, rc, s);
+        int launched = 0;
+        st = run_resident_jobs(jobs.data(), n, ckpt_every, bufs[0].pb / sizeof(float), nullptr, rc, s, &launched);
         if (st != HS_ERR_UNSUPPORTED) return st;
+        pairs += launched;
+        bufs += launched;
+        n -= launched;
     }
     for (int i = 0; i < n; ++i) {
         const hs_train_pair &d = pairs[i];

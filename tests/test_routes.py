@@ -109,3 +109,43 @@ def test_training_forward_with_an_output_over_another_pairs_image(fake):
     assert "derivs_kernel" in ks and "hs_resident_kernel" not in ks
     fake.reset()
     assert "hs_resident_kernel" in kernels(train(fake, [(H, W)] * 2, 20, 5, planes=apart))
+
+
+# ------------------------------------------------------------------ fewer SMs than the device has
+
+def in_place(n):
+    """Pairs whose flow takes the place of their images."""
+    at = [((1 << 36) + 2 * i * 64 * MB, (1 << 36) + (2 * i + 1) * 64 * MB) for i in range(n)]
+    return [(a, b, a, b) for a, b in at]
+
+
+def refused_from(ls, planes):
+    """The first pair of the first refused launch, after at least one that was made."""
+    ls = [x for x in ls if x.kernel == "hs_resident_kernel"]
+    assert [x.refused for x in ls[:2]] == [False, True]
+    return [at[0] for at in planes].index(ls[1].first)
+
+
+def test_batch_redoes_only_what_was_not_launched(fake):
+    """Two launches of different size on a device that holds the first one's tiles only: the pairs
+    of the first have their flow where their images were, and are not read again."""
+    specs = [(500, 700, 40)] * 6 + [(900, 1300, 30)]
+    planes = in_place(len(specs))
+    tiles = [x.grid for x in batch(fake, specs, planes=planes) if x.kernel == "hs_resident_kernel"]
+    assert len(tiles) == 2 and tiles[0] < tiles[1]
+    fake.reset(max_cooperative_blocks=tiles[0])
+    ls = batch(fake, specs, planes=planes)
+    k = refused_from(ls, planes)
+    again = [x.first for x in ls if not x.refused and x.kernel in ("derivs_kernel", "hs_resident_kernel")][1:]
+    assert k > 0 and again == [at[0] for at in planes[k:]]
+
+
+def test_training_forward_redoes_only_what_was_not_launched(fake):
+    shapes = [(500, 700)] * 6 + [(900, 1300)]
+    planes = in_place(len(shapes))
+    tiles = [x.grid for x in train(fake, shapes, 40, 10, planes=planes) if x.kernel == "hs_resident_kernel"]
+    assert len(tiles) == 2 and tiles[0] < tiles[1]
+    fake.reset(max_cooperative_blocks=tiles[0])
+    ls = train(fake, shapes, 40, 10, planes=planes)
+    k = refused_from(ls, planes)
+    assert k > 0 and [x.first for x in ls if x.kernel == "derivs_kernel"] == [at[0] for at in planes[k:]]

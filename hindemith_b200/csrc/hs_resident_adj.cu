@@ -5,7 +5,7 @@
 // to three adjoint passes over all images; on small images those are launches, on large ones every
 // pass moves lambda, the coefficients and the accumulators.  Here a tile per SM keeps them: the
 // coefficients in tensor memory, lambda (or the recomputed state) in registers, the accumulators
-// dIx, dIy, dIt of an interval in shared memory.  Per interval, from the last:
+// dIx, dIy, dIt of a few sweeps in shared memory.  Per interval, from the last:
 //   1. the states of its inner sweeps are recomputed from its checkpoint (the resident sweep, with
 //      an exchange every kResT sweeps) and written to the interval's state buffer;
 //   2. lambda comes back, and the interval's sweeps are reversed: M pointwise (hs_train.cu's
@@ -14,9 +14,10 @@
 //      states before their reads in the halo.  The state buffers alternate by interval parity: a
 //      neighbour still reading interval b's is done before this tile, having received its
 //      messages of interval b-1, writes b-2's;
-//   3. the interval's accumulators are added to the planes in global memory, and lambda is parked
-//      there.  (Sums of one interval's terms, then the sum over intervals: no longer chains of
-//      additions than the streaming passes have.)
+//   3. lambda is parked in global memory.
+// Every `chain` sweeps, whatever the intervals, the accumulators are added to the planes in global
+// memory: chains of `chain` terms and then one of iters / chain sums, where the streaming passes
+// have chains of 4 and one of iters / 4.
 // The arithmetic of a cell is the streaming kernels'.
 #include <algorithm>
 #include <cstring>
@@ -49,6 +50,7 @@ struct ResAdjTable {
     unsigned *abort_flag;
     size_t plane;                // floats between planes
     int ckpt_every, iters, nslots;
+    int chain;                   // sweeps whose terms are summed before they join the planes
     float we, wc;
 };
 
@@ -80,7 +82,7 @@ __device__ __forceinline__ void adj_fetch(const ResLane &t, const ResTile &g, in
 
 // One sweep's M on the warp's rows: lambda -> z in place; x: the state after the sweep (planes xu,
 // xu + plane), its first rows already in q; next: the state the next call works from, whose first
-// rows are loaded into q (or null); acc: the interval's accumulators, of own cells; a2: the lane's
+// rows are loaded into q (or null); acc: the accumulators, of own cells; a2: the lane's
 // columns' sums of lr (-t).
 template <bool FAST, int R>
 __device__ __forceinline__ void adj_rows(const ResLane &t, const ResTile &g, float2 (&cu)[R][2][2],
@@ -198,9 +200,32 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 1) hs_resident_adj_kernel(cons
         }
         __syncwarp();
     };
+    // the accumulators join the planes in global memory (each thread its own cells; the first ones
+    // are the planes' start).  Called before a sweep, not after it: the sweep's registers are dead
+    // there (after it R = 5 spilled twice as much, 2 x 700^2 x 200 1.96 -> 2.08 ms).
+    auto flush = [&](bool first) {
+#pragma unroll 1
+        for (int r = 0; r < R; ++r) {
+            const int row = t.row0 + r;
+            if (!(g.own_col && row >= g.y0 && row < g.y1)) continue;
+            const size_t off = (size_t)row * p.ld + g.xa;
+            for (int i = 0; i < 3; ++i) {
+                float4 *a = reinterpret_cast<float4 *>(p.acc + i * pl + off);
+                float4 *s = acc + (i * A::rows + row - g.y0) * kResChunks + (lane - 1);
+                float4 v = *s;
+                if (!first) {
+                    const float4 w = *a;
+                    v = make_float4(w.x + v.x, w.y + v.y, w.z + v.z, w.w + v.w);
+                }
+                *a = v;
+                *s = z4;
+            }
+        }
+        __syncwarp();
+    };
     unsigned e = 0;
-    int half = 0;
-    bool ok = true;
+    int half = 0, left = tab.chain;  // left: sweeps until the accumulators join the planes
+    bool first = true, ok = true;
     double a2sum = 0.0;
     for (int b = nb - 1; b >= 0 && ok; --b) {
         const int nsw = min(k, tab.iters - b * k);
@@ -229,6 +254,12 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 1) hs_resident_adj_kernel(cons
 #pragma unroll
         for (int r = 0; r < adj_ahead<R>(); ++r) adj_fetch(t, g, r, state_of(nsw), state_of(nsw) + pl, xq[r]);
         for (int m = nsw; m >= 1; --m) {
+            if (left == 0) {
+                flush(first);
+                first = false;
+                left = tab.chain;
+            }
+            --left;
             if ((nsw - m) % kResT == 0 && tiles > 1) {
                 ok = m == nsw ? res_exchange<NW, R, true>(t, g, cu, out, in, src, p.box, ++e, &stop, tab.abort_flag, nullptr)
                               : res_exchange<NW, R, false>(t, g, cu, out, in, src, p.box, ++e, &stop, tab.abort_flag, nullptr);
@@ -247,25 +278,8 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 1) hs_resident_adj_kernel(cons
             half ^= 1;
         }
         if (!ok) break;
-        // 3. the accumulators to global memory, lambda parked (each thread its own cells)
-#pragma unroll 1
-        for (int r = 0; r < R; ++r) {
-            const int row = t.row0 + r;
-            if (!(g.own_col && row >= g.y0 && row < g.y1)) continue;
-            const size_t off = (size_t)row * p.ld + g.xa;
-            for (int i = 0; i < 3; ++i) {
-                float4 *a = reinterpret_cast<float4 *>(p.acc + i * pl + off);
-                float4 *s = acc + (i * A::rows + row - g.y0) * kResChunks + (lane - 1);
-                float4 v = *s;
-                if (b != nb - 1) {
-                    const float4 w = *a;
-                    v = make_float4(w.x + v.x, w.y + v.y, w.z + v.z, w.w + v.w);
-                }
-                *a = v;
-                *s = z4;
-            }
-        }
-        __syncwarp();
+        if (b == 0) flush(first);  // (left < chain: at least one sweep is in them)
+        // 3. lambda parked (each thread its own cells)
         if (b > 0) res_store_own<R>(t, g, cu, p.park, p.park + pl);
     }
     __syncthreads();
@@ -379,6 +393,11 @@ hs_status run_resident_adjoint(const ResidentAdjJob *jobs, int n, int iters, int
         tab.plane = plane;
         tab.ckpt_every = ckpt_every;
         tab.iters = iters;
+        // Terms of like size, FP32 on the CPU against 64 bits, relative error of the sums in 1e-8 (the
+        // passes' order, chains of 4 / this one / one chain per checkpoint interval of all sweeps):
+        // 16 sweeps 4.2 / 4.2 / 6.1, 50 sweeps 5.8 / 4.8 / 10.4, 200 sweeps 10.5 / 5.9 / 20.6.  (An
+        // interval each instead: 600x800, 100 sweeps, intervals of 1, 977 us against 727.)
+        tab.chain = iters < 32 ? 4 : iters < 64 ? 8 : 16;
         tab.nslots = nslots;
         tab.we = rc.we;
         tab.wc = rc.wc;

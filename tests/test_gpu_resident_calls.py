@@ -40,3 +40,69 @@ def test_forward_writing_inside_its_images_memory(cuda, fast, rows):
         D.hs_forward(a, I1, 1.0, 40, cfg, out=(u, v))
         equal(u, ru, "u")
         equal(v, rv, "v")
+
+
+# ------------------------------------------------------------------ the backward's sums
+
+class SinglePair:
+    """hs_forward_train and hs_backward on buffers of the test's own, whose parts it reads."""
+
+    def __init__(self, H, W, iters, ckpt, cfg, seed):
+        import ctypes
+
+        self.lib, self.cfg, self.ct = L.lib(), ctypes.byref(cfg), ctypes
+        self.H, self.W, self.ld, self.iters, self.ckpt = H, W, (W + 3) // 4 * 4, iters, ckpt
+        self.I0, self.I1 = images((H, W), 2, seed)
+        self.stride = (H * self.ld * 4 + 255) // 256 * 256
+        self.alpha = torch.tensor([0.9], device="cuda")
+        u, v = images((H, W), 2, 0)
+        nd = self.lib.hs_derivs_bytes(H, W, self.ld)
+        nc = self.lib.hs_checkpoint_bytes(H, W, self.ld, iters, ckpt)
+        nw = self.lib.hs_forward_train_workspace_bytes(H, W, self.ld)
+        self.derivs, self.planes, ws = (torch.zeros(n, dtype=torch.uint8, device="cuda") for n in (nd, nc, nw))
+        L.check(self.lib.hs_forward_train(D.ptr(self.I0), D.ptr(self.I1), H, W, self.ld, D.ptr(self.alpha), iters, ckpt,
+                                          D.ptr(u), D.ptr(v), D.ptr(self.derivs), D.ptr(self.planes), D.ptr(ws), nw,
+                                          self.cfg, D.stream_handle()), "hs_forward_train")
+
+    def plane(self, buf, k):
+        b = buf[k * self.stride:k * self.stride + self.H * self.ld * 4].view(torch.float32)
+        return b.view(self.H, self.ld)[:, :self.W]
+
+    def backward(self, first, intervals, iters, ckpt, lu, lv):
+        """The sweeps from checkpoint plane `first` on; (accumulators, lambda parked before the first
+        interval)."""
+        need = self.lib.hs_backward_workspace_bytes(self.H, self.W, self.ld, ckpt)
+        ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+        out = images((self.H, self.W), 2, 0)
+        da = torch.zeros(1, device="cuda")
+        at = self.ct.c_void_p(self.planes.data_ptr() + 2 * first * self.stride)
+        L.check(self.lib.hs_backward(D.ptr(self.derivs), self.H, self.W, self.ld, D.ptr(self.alpha), iters, ckpt, at, D.ptr(lu),
+                                     D.ptr(lv), D.ptr(out[0]), D.ptr(out[1]), D.ptr(da), D.ptr(ws), need, self.cfg,
+                                     D.stream_handle()), "hs_backward")
+        lam = 4 * (ckpt - 1)
+        return ([self.plane(ws, lam + 4 + i).clone() for i in range(3)],
+                [D.as_plane(self.plane(ws, lam + i).clone()) for i in range(2)])
+
+
+@pytest.mark.parametrize("ckpt", [1, 100])
+def test_backward_sums_no_further_off_than_the_passes_order(cuda, ckpt):
+    """dIx, dIy, dIt over 100 sweeps: the same terms as 25 backwards of 4 sweeps each.  Against
+    these added in 64 bits, the sums of one call are no further off than these added in 32 bits one
+    after the other, the order of the streaming passes (10 % for the sample)."""
+    H, W, n = 600, 800, 100
+    cfg = L.make_config(fast_math=True)
+    lam = images((H, W), 2, 7)
+    four = SinglePair(H, W, n, 4, cfg, 3)
+    one = SinglePair(H, W, n, ckpt, cfg, 3)
+    got, _ = one.backward(0, n // ckpt, n, ckpt, *lam)
+    sum64, sum32 = [0.0] * 3, None
+    l = lam
+    for c in range(n // 4 - 1, -1, -1):
+        acc, _ = four.backward(c, 1, 4, 4, *l)
+        sum64 = [s + a.double() for s, a in zip(sum64, acc)]
+        sum32 = [s + a for s, a in zip(sum32, acc)] if sum32 else acc
+        if c:
+            l = four.backward(c - 1, 2, 8, 4, *l)[1]
+    for k in range(3):
+        off = [float((s.double() - sum64[k]).norm()) for s in (got[k], sum32[k])]
+        assert off[0] <= 1.1 * off[1], (k, off)

@@ -212,9 +212,10 @@ size_t resident_box_bytes(int tiles, int r) {
 // outboxes fit the scratch.
 bool resident_plan(int H, int W, int iters, size_t scratch_bytes, ResidentPlan &pl) {
     if (iters < 2) return false;
+    const int sms = sm_count();
     for (int r = kResMinR; r <= kResMaxR; ++r) {
         const int tiles = resident_tiles(H, W, r, &pl.ntx, &pl.nty);
-        if (tiles > sm_count()) continue;
+        if (tiles > sms) continue;
         pl.r = r;
         pl.box_bytes = resident_box_bytes(tiles, r);
         if (pl.box_bytes <= scratch_bytes) return true;
@@ -298,16 +299,25 @@ bool resident_cut(const ResidentJob *jobs, int n, double base, double slope, int
     std::vector<double> cost(n + 1, -1.0);
     std::vector<int> from(n + 1, 0), rows(n + 1, 0);
     cost[0] = 0.0;
+    // the tiles of every job at every height, formed once (n^2 of them, each asking for the device,
+    // made 900 us of host time for 64 images); one more than the SMs where it does not fit
+    const int sms = sm_count();
+    std::vector<int> need((size_t)n * (max_r + 1));
+    for (int j = 0; j < n; ++j)
+        for (int r = kResMinR; r <= max_r; ++r) {
+            int ntx, nty;
+            const int t = resident_tiles(jobs[j].H, jobs[j].W, r, &ntx, &nty);
+            need[(size_t)j * (max_r + 1) + r] =
+                t <= sms && resident_box_bytes(t, r) <= jobs[j].scratch_bytes ? t : sms + 1;
+        }
     for (int i = 0; i < n; ++i) {  // a launch that starts with job i
         if (cost[i] < 0.0) continue;
         for (int r = kResMinR; r <= max_r; ++r) {
             const double sweep = base + slope * r;
             int tiles = 0, longest = 0;
             for (int j = i; j < n && j < i + kMaxResImages; ++j) {
-                int ntx, nty;
-                const int t = resident_tiles(jobs[j].H, jobs[j].W, r, &ntx, &nty);
-                tiles = std::min(tiles + std::min(t, sm_count() + 1), sm_count() + 1);
-                if (tiles > sm_count() || resident_box_bytes(t, r) > jobs[j].scratch_bytes) break;
+                tiles += need[(size_t)j * (max_r + 1) + r];
+                if (tiles > sms) break;
                 longest = std::max(longest, jobs[j].iters);
                 const double c = cost[i] + sweep * longest + 8.0;  // (and about 8 us for a launch)
                 if (cost[j + 1] < 0.0 || c < cost[j + 1]) {

@@ -12,6 +12,7 @@ static int nkernels;
 static char *text;
 static size_t len, cap;
 static int coop_limit = 1 << 30; /* cooperative launches of more blocks are refused */
+static int queries; /* calls that ask for the device or an attribute */
 
 static void record(const char *fmt, ...) {
     va_list ap;
@@ -28,10 +29,12 @@ static const char *name_of(const void *host) {
 
 void fake_reset(int max_cooperative_blocks) {
     len = 0;
+    queries = 0;
     coop_limit = max_cooperative_blocks;
     record("%s", "");
 }
 const char *fake_log(void) { return text ? text : ""; }
+int fake_queries(void) { return queries; }
 
 /* registration and launches */
 void **__cudaRegisterFatBinary(void *p) { static void *h; (void)p; return &h; }
@@ -91,7 +94,7 @@ cudaError_t cudaMemcpy2DAsync(void *d, size_t dp, const void *p, size_t sp, size
     (void)dp; (void)sp;
     return cudaMemcpyAsync(d, p, w * h, k, s);
 }
-cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaGetDevice(int *d) { ++queries; *d = 0; return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int *v, enum cudaDeviceAttr a, int d) {
     (void)d;
     *v = a == cudaDevAttrMultiProcessorCount ? 148 : a == cudaDevAttrComputeCapabilityMajor ? 10 : 0;

@@ -149,3 +149,18 @@ def test_training_forward_redoes_only_what_was_not_launched(fake):
     ls = train(fake, shapes, 40, 10, planes=planes)
     k = refused_from(ls, planes)
     assert k > 0 and [x.first for x in ls if x.kernel == "derivs_kernel"] == [at[0] for at in planes[k:]]
+
+
+# ------------------------------------------------------------------ host work of a batch
+
+@pytest.mark.parametrize("n,H,W", [(64, 64, 64), (128, 240, 320)])
+def test_batch_planning_asks_for_the_device_a_few_times_per_pair(fake, n, H, W):
+    batch(fake, [(H, W, 100)] * n)
+    assert fake.lib.fake_queries() <= 8 * n
+
+
+def test_training_planning_asks_for_the_device_a_few_times_per_pair(fake):
+    for backward in (False, True):
+        fake.reset()
+        train(fake, [(128, 128)] * 32, 50, 5, backward=backward)
+        assert fake.lib.fake_queries() <= 8 * 32

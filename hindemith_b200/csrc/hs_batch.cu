@@ -418,18 +418,28 @@ hs_status hs_forward_batched(const hs_pair_desc *pairs, int n, void *workspace,
     int *status = device_status ? device_status : reinterpret_cast<int *>(ws + 4);
     unsigned *abort_flag = reinterpret_cast<unsigned *>(ws + 8);
 
+    if (device_status) HS_CUDA_CHECK(cudaMemsetAsync(device_status, 0, sizeof(int), s));
+
     // No depth, tile or layout asked for: the images that fit the chip run there (hs_resident.cuh),
-    // longest first, as many at a time as the SMs hold, and each larger one in its own passes.  The
-    // persistent kernel below serves explicit settings: its chains of dependent passes leave the
+    // longest first, as many at a time as the SMs hold, and each larger one in its own passes.
+    // The persistent kernel below serves explicit settings: its chains of dependent passes leave the
     // chip idle unless many tiles are independent (measured on B200, fast form, Gpix-it/s, at its
     // default depth 4 -> this way: 16 mixed pairs 545 -> 672, 3 of 2048^2 528 -> 649, 8 of 640x480
-    // 185 -> 628, 12 of 320x240 84 -> 474).
-    if (wants_resident(rc) && outputs_apart(pairs, n)) {
-        if (device_status) HS_CUDA_CHECK(cudaMemsetAsync(device_status, 0, sizeof(int), s));
-        std::vector<int> in;
-        for (int i = 0; i < n; ++i)
-            if (resident_fits(pairs[i].H, pairs[i].W, pairs[i].iters, 5 * round_up(plane_bytes(pairs[i].H, pairs[i].ld), 256)))
-                in.push_back(i);
+    // 185 -> 628, 12 of 320x240 84 -> 474).  The rest goes there too: pairs of no sweep or one,
+    // images below 1.5 Mpx that cut into more tiles than SMs for their shape, or whose exchange does
+    // not fit their scratch.  In calls of their own these are launches and half-empty passes (64
+    // pairs of 16x16 without a sweep 395 us against 8, of 64x64 with one 485 against 221; 12 of
+    // 3x3000 x 100 1089 against 186, of 8x20000 x 40 760 against 274; 4 of 50x20000 517 against 500
+    // fast, 808 against 934 exact, 2 of 90x20000 342 against 627).
+    std::vector<char> done(n, 0), apart(n, 0);  // apart: in a call of its own
+    std::vector<int> in;
+    if (wants_resident(rc))
+        for (int i = 0; i < n; ++i) {
+            const hs_pair_desc &d = pairs[i];
+            if (resident_fits(d.H, d.W, d.iters, 5 * round_up(plane_bytes(d.H, d.ld), 256))) in.push_back(i);
+            else apart[i] = d.iters >= 2 && (long)d.H * d.W >= 1500000;
+        }
+    if ((!in.empty() || std::count(apart.begin(), apart.end(), 1)) && outputs_apart(pairs, n)) {
         std::sort(in.begin(), in.end(), [&](int a, int b) {
             return pairs[a].iters != pairs[b].iters ? pairs[a].iters > pairs[b].iters : a < b;
         });
@@ -449,21 +459,23 @@ hs_status hs_forward_batched(const hs_pair_desc *pairs, int n, void *workspace,
         int launched = 0;
         st = run_resident_jobs(jobs.data(), (int)jobs.size(), 0, 0, device_status, rc, s, &launched);
         if (st != HS_OK && st != HS_ERR_UNSUPPORTED) return st;
-        std::vector<char> done(n, 0);
-        for (int k = 0; k < launched; ++k) done[in[k]] = 1;
+        for (int k = 0; k < (int)in.size(); ++k) (k < launched ? done : apart)[in[k]] = 1;
         for (int i = 0; i < n; ++i) {
             const hs_pair_desc &d = pairs[i];
-            if (done[i]) continue;
+            if (!apart[i]) continue;
+            done[i] = 1;
             if ((st = hs_forward(d.I0, d.I1, d.H, d.W, d.ld, d.alpha, d.iters, d.u, d.v, ws + plan[i].off_planes,
                                  5 * round_up(plane_bytes(d.H, d.ld), 256), cfg, stream)) != HS_OK)
                 return st;
         }
-        return HS_OK;
     }
+    std::vector<int> rest;
+    for (int i = 0; i < n; ++i)
+        if (!done[i]) rest.push_back(i);
+    if (rest.empty()) return HS_OK;
 
     // header and every pair's tile-progress counters start at zero
     HS_CUDA_CHECK(cudaMemsetAsync(ws, 0, kHeaderBytes, s));
-    if (device_status) HS_CUDA_CHECK(cudaMemsetAsync(device_status, 0, sizeof(int), s));
     const size_t prog_begin = plan.front().off_progress;
     HS_CUDA_CHECK(cudaMemsetAsync(ws + prog_begin, 0, total - prog_begin, s));
 
@@ -471,9 +483,10 @@ hs_status hs_forward_batched(const hs_pair_desc *pairs, int n, void *workspace,
     std::vector<BatchPair> bpairs(n);
     DerivParams dp;
     memset(&dp, 0, sizeof(dp));
-    dp.npairs = n;
+    dp.npairs = (int)rest.size();
     int maxW = 1, maxH = 1;
-    for (int i = 0; i < n; ++i) {
+    for (int r = 0; r < dp.npairs; ++r) {
+        const int i = rest[r];
         const PairPlan &p = plan[i];
         const hs_pair_desc &d = pairs[i];
         const size_t pb = round_up(plane_bytes(p.H, p.ld), 256);
@@ -496,22 +509,22 @@ hs_status hs_forward_batched(const hs_pair_desc *pairs, int n, void *workspace,
         b.nstrips = p.nstrips;
         b.seg_rows = p.seg_rows;
         b.items = p.items;
-        dp.I0[i] = d.I0;
-        dp.I1[i] = d.I1;
-        dp.Ix[i] = const_cast<float *>(b.Ix);
-        dp.Iy[i] = const_cast<float *>(b.Iy);
-        dp.It[i] = const_cast<float *>(b.It);
-        dp.U0[i] = b.U[p.start];
-        dp.V0[i] = b.V[p.start];
-        dp.H[i] = p.H;
-        dp.W[i] = p.W;
-        dp.ld[i] = p.ld;
+        dp.I0[r] = d.I0;
+        dp.I1[r] = d.I1;
+        dp.Ix[r] = const_cast<float *>(b.Ix);
+        dp.Iy[r] = const_cast<float *>(b.Iy);
+        dp.It[r] = const_cast<float *>(b.It);
+        dp.U0[r] = b.U[p.start];
+        dp.V0[r] = b.V[p.start];
+        dp.H[r] = p.H;
+        dp.W[r] = p.W;
+        dp.ld[r] = p.ld;
         maxW = std::max(maxW, p.W);
         maxH = std::max(maxH, p.H);
     }
     {
         dim3 block(64, 4);
-        dim3 grid((unsigned)((maxW + 63) / 64), (unsigned)((maxH + 3) / 4), (unsigned)n);
+        dim3 grid((unsigned)((maxW + 63) / 64), (unsigned)((maxH + 3) / 4), (unsigned)dp.npairs);
         batch_derivs_kernel<<<grid, block, 0, s>>>(dp);
         HS_LAUNCH_CHECK("batch_derivs_kernel");
     }
@@ -521,7 +534,7 @@ hs_status hs_forward_batched(const hs_pair_desc *pairs, int n, void *workspace,
     for (int lay = 1; lay >= 0; --lay) {
         const bool wide = lay == 1;
         std::vector<int> members;
-        for (int i = 0; i < n; ++i)
+        for (int i : rest)
             if (plan[i].wide == wide && bpairs[i].passes > 0) members.push_back(i);
         if (members.empty()) continue;
         const int m = (int)members.size();
@@ -552,7 +565,7 @@ hs_status hs_forward_batched(const hs_pair_desc *pairs, int n, void *workspace,
     }
 
     // the short last pass of pairs whose sweep count is not a multiple of T
-    for (int i = 0; i < n; ++i) {
+    for (int i : rest) {
         const PairPlan &p = plan[i];
         if (p.rem == 0) continue;
         const BatchPair &b = bpairs[i];

@@ -106,3 +106,45 @@ def test_backward_sums_no_further_off_than_the_passes_order(cuda, ckpt):
     for k in range(3):
         off = [float((s.double() - sum64[k]).norm()) for s in (got[k], sum32[k])]
         assert off[0] <= 1.1 * off[1], (k, off)
+
+
+# ------------------------------------------------------------------ the batched call's default
+
+MIXED = [(1, 1, 1.0, 3), (7, 130, 0.5, 9), (65, 127, 1.7, 40), (300, 518, 0.8, 37), (130, 7, 1.2, 0), (240, 320, 2.0, 100),
+         (480, 640, 0.6, 23), (33, 65, 1.0, 8), (200, 90, 0.9, 1), (3, 3000, 1.1, 9), (25, 121, 1.0, 2)]
+BATCHES = {
+    "mixed": MIXED,
+    "with an image above 2 Mpx": MIXED[:4] + [(1100, 1925, 0.7, 9)] + MIXED[4:],
+    "more than 32 small images": [(20 + 3 * k, 30 + 7 * k, 1.0, 4 + k % 5) for k in range(40)],
+    "several launches": [(500, 701, 1.0, 12)] * 6 + [(900, 1301, 0.8, 7), (720, 1280, 1.3, 9)],
+    "no sweep or one": [(40, 52, 1.0, 0), (41, 53, 1.0, 1)] * 5,
+}
+
+
+@pytest.mark.parametrize("fast", [True, False])
+@pytest.mark.parametrize("name", list(BATCHES))
+def test_batch_by_default_equals_per_pair_passes(cuda, name, fast):
+    """Eager and as a replayed graph, into outputs full of NaN."""
+    from hindemith_b200.batched import BatchPlan
+
+    specs = BATCHES[name]
+    plan = BatchPlan(specs, L.make_config(fast_math=fast))
+    refs = []
+    for i, (H, W, alpha, iters) in enumerate(specs):
+        for t, x in zip((plan.I0[i], plan.I1[i]), images((H, W), 2, 100 + i)):
+            t.copy_(x)
+        refs.append(D.hs_forward(plan.I0[i], plan.I1[i], alpha, iters, L.make_config(fast_math=fast, sweeps_per_pass=3, layout=1)))
+
+    def run(go):
+        for t in plan.u + plan.v:
+            t.fill_(float("nan"))
+        go()
+        plan.check()
+        for i, (ru, rv) in enumerate(refs):
+            equal(plan.u[i], ru, f"u of pair {i}")
+            equal(plan.v[i], rv, f"v of pair {i}")
+
+    run(plan.run)
+    plan.capture()
+    for _ in range(2):
+        run(plan.replay)

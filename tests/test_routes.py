@@ -164,3 +164,28 @@ def test_training_planning_asks_for_the_device_a_few_times_per_pair(fake):
         fake.reset()
         train(fake, [(128, 128)] * 32, 50, 5, backward=backward)
         assert fake.lib.fake_queries() <= 8 * 32
+
+
+# ------------------------------------------------------------------ pairs that do not run on the chip
+
+@pytest.mark.parametrize("specs,most", [([(16, 16, 0)] * 64, 1), ([(64, 64, 1)] * 64, 1 + 64),
+                                        ([(3, 3000, 9)] * 12, 3 + 12), ([(8, 20000, 8)] * 12, 3),
+                                        ([(240, 320, 50), (64, 64, 0), (300, 400, 1), (2200, 2000, 14)], 2 + 3 + 2)])
+def test_batch_of_pairs_without_a_resident_form_shares_its_launches(fake, specs, most):
+    """No sweep or one, images whose exchange their scratch does not hold or whose shape cuts into
+    more tiles than SMs: one derivative launch and the persistent kernel for all of them, and a
+    launch per remainder of the depth."""
+    ls = batch(fake, specs)
+    assert len(ls) <= most
+    assert sum(x.kernel == "batch_derivs_kernel" for x in ls) == 1
+    assert sum(x.kernel == "derivs_kernel" for x in ls) == sum(H * W > 4e6 for H, W, _ in specs)
+
+
+def test_batch_of_large_pairs_and_small_ones_does_each_once(fake):
+    """Every pair in exactly one of the three ways."""
+    specs = [(2200, 2000, 14), (240, 320, 50), (3, 3000, 9), (16, 16, 0)]
+    ls = batch(fake, specs)
+    at = [(1 << 36) + 4 * i * 64 * MB for i in range(4)]
+    assert [x.first for x in ls if x.kernel == "derivs_kernel"] == at[:1]
+    assert [x.first for x in ls if x.kernel == "hs_resident_kernel"] == at[1:2]
+    assert [x.first for x in ls if x.kernel == "batch_derivs_kernel"] == at[2:3]

@@ -588,7 +588,7 @@ hs_status hs_forward_batched(const hs_pair_desc *pairs, int n, void *workspace,
         pp.wc = rc.wc;
         const int sc = strip_cols_for(p.rem);
         pp.nstrips = (p.W + sc - 1) / sc;
-        pp.seg_rows = default_seg_rows(p.H, pp.nstrips, p.rem);
+        pp.seg_rows = default_seg_rows(p.H, pp.nstrips, p.rem, rc.fast);
         pp.nitems = pp.nstrips * ((p.H + pp.seg_rows - 1) / pp.seg_rows);
         if ((st = launch_pass(p.rem, rc.fast, pp, s)) != HS_OK) return st;
     }

@@ -33,6 +33,7 @@
 #pragma once
 
 #include <algorithm>
+#include <atomic>
 #include <vector>
 
 #include "hs_common.cuh"
@@ -413,7 +414,10 @@ hs_status resolve_config(const hs_config *cfg, ResolvedConfig *out);
 // for the per-pair sweep: when no depth was given, the measured default for an H x W image
 void apply_shape_default(ResolvedConfig &rc, int H, int W);
 int strip_cols_for(int T);
-int default_seg_rows(int H, int nstrips, int T);
+int default_seg_rows(int H, int nstrips, int T, bool fast);
+// Warps of a kernel, in CTAs of `warps`, that an SM holds at once; `cache` (one entry per device, 0 at
+// first) keeps the answer.
+int held_warps(const void *kernel, int warps, size_t smem, std::atomic<int> *cache);
 hs_status launch_pass(int T, bool fast, const SweepParams &pp, cudaStream_t s);
 // `iters` sweeps; the state starts in (u0, v0) for an even number of passes, in (u1, v1)
 // for an odd one, and always ends in (u0, v0).  alpha_dev, if set, overrides alpha2.

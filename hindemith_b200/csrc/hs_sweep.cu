@@ -115,6 +115,46 @@ static hs_status launch_kernel(KernelFn fn, int smem, bool *attr_set, const Swee
 // in tensor memory, 2043x1543 528 against 511, 1700x2000 601 against 610).
 constexpr long kTmPixels = 3300000;
 
+int held_warps(const void *kernel, int warps, size_t smem, std::atomic<int> *cache) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 0;
+    int held = cache[dev].load(std::memory_order_relaxed);
+    if (held == 0) {
+        int ctas = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, kernel, warps * 32, smem) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        held = ctas * warps;
+        cache[dev].store(held, std::memory_order_relaxed);
+    }
+    return held;
+}
+
+// Warps of a pass's kernel that an SM holds at once (its launch bound is the least it may hold).
+template <int T>
+static int pass_warps_at(bool fast) {
+    static std::atomic<int> held[2][64];
+    constexpr size_t smem = kPassWarps * Geo<T>::warp_floats * sizeof(float);
+    const int h = fast ? held_warps((const void *)hs_stream_kernel<T, true, (T <= 2)>, kPassWarps, smem, held[1])
+                       : held_warps((const void *)hs_stream_kernel<T, false, (T <= 2)>, kPassWarps, smem, held[0]);
+    return std::max(h, res_warps(T));
+}
+template <int T>
+static int pass_warps_w_at(bool tm) {
+    static std::atomic<int> held[2][64];
+    const int h = tm ? held_warps((const void *)hs_stream_tm_kernel<T>, kTmWarps, 0, held[1])
+                     : held_warps((const void *)hs_stream_w_kernel<T>, kPassWarps,
+                                  kPassWarps * GeoW<T>::warp_floats * sizeof(float), held[0]);
+    return std::max(h, res_warps_w(T));
+}
+#define HS_BY_DEPTH(F, T, ARG)                                                            \
+    ((T) == 1 ? F<1>(ARG) : (T) == 2 ? F<2>(ARG) : (T) == 3 ? F<3>(ARG) : (T) == 4 ? F<4>(ARG) \
+     : (T) == 5 ? F<5>(ARG) : (T) == 6 ? F<6>(ARG) : (T) == 7 ? F<7>(ARG) : F<8>(ARG))
+static int pass_warps(int T, bool fast) { return HS_BY_DEPTH(pass_warps_at, T, fast); }
+static int pass_warps_w(int T, bool tm) { return HS_BY_DEPTH(pass_warps_w_at, T, tm); }
+#undef HS_BY_DEPTH
+
 template <int T>
 static hs_status launch_one_w(const SweepParams &pp, cudaStream_t stream) {
     if ((long)pp.H * pp.W < kTmPixels) {
@@ -215,20 +255,28 @@ hs_status launch_pass(int T, bool fast, const SweepParams &pp, cudaStream_t s) {
     HS_FAIL(HS_ERR_INVALID_ARG, "sweeps_per_pass=%d outside 1..%d", T, HS_MAX_SWEEPS_PER_PASS);
 }
 
-// Rows per work item: as many items as the SMs hold at once and not one more (a single item in a
-// second wave costs the pass nearly half as much again: 3840x2160, T = 6, 1190 items for 1184
-// slots 581 Gpix-it/s, 1155 items 791; 2048^2 643 -> 695), but never so few rows that the 2T-row
-// halo dominates.
-static int seg_rows_for(int H, int nstrips, int T, long warps_per_sm) {
-    const long target = (long)sm_count() * warps_per_sm;
-    const long nseg = std::max(1L, target / nstrips);
-    int L = (int)((H + nseg - 1) / nseg);
-    L = std::max(L, 2 * T);
-    L = std::max(L, 8);
-    return std::min(L, H);
+// Rows per work item: items for about `want` warps per SM, but not one more than the SMs hold at once
+// (`held` per SM): a single item in a second wave costs the pass nearly half as much again
+// (3840x2160, T = 6, 1190 items for 1184 slots 581 Gpix-it/s, 1155 items 791; 2048^2 643 -> 695).
+// Never so few rows that the 2T-row halo dominates.  (What is held is more than the launch bound
+// where a kernel needs fewer registers: the 2-column fast form holds 19 warps at T = 5, and cutting
+// it for 12 takes 1811x2048 from 143 to 181 us for 20 sweeps.)
+static int seg_rows_for(int H, int nstrips, int T, long want, long held) {
+    const long slots = (long)sm_count() * held;
+    auto rows = [&](long nseg) {
+        int L = (int)((H + nseg - 1) / nseg);
+        L = std::max(L, 2 * T);
+        L = std::max(L, 8);
+        return std::min(L, H);
+    };
+    const int L = rows(((long)sm_count() * want + nstrips - 1) / nstrips);
+    if ((long)nstrips * ((H + L - 1) / L) <= slots) return L;
+    return rows(std::max(1L, slots / nstrips));
 }
 
-int default_seg_rows(int H, int nstrips, int T) { return seg_rows_for(H, nstrips, T, res_warps(T)); }
+int default_seg_rows(int H, int nstrips, int T, bool fast) {
+    return seg_rows_for(H, nstrips, T, 16, pass_warps(T, fast));
+}
 
 // Measured on B200: in a launch of several pairs (the batch and the training passes) the wide
 // layout wins from about a 1080p image up (4096^2: 700 vs 592 Gpix-it/s), the narrow one below
@@ -315,7 +363,8 @@ hs_status run_passes_dev(const float *Ix, const float *Iy, const float *It, int 
         const int sc = wide ? strip_cols_wide(t) : strip_cols_for(t);
         pp.nstrips = (W + sc - 1) / sc;
         pp.seg_rows = rc.seg_rows > 0 ? std::min(rc.seg_rows, H)
-                                      : seg_rows_for(H, pp.nstrips, t, wide ? res_warps_w(t) : res_warps(t));
+                      : wide ? seg_rows_for(H, pp.nstrips, t, res_warps_w(t), pass_warps_w(t, (long)H * W >= kTmPixels))
+                             : default_seg_rows(H, pp.nstrips, t, rc.fast);
         const int nseg = (H + pp.seg_rows - 1) / pp.seg_rows;
         pp.nitems = pp.nstrips * nseg;
         hs_status st = wide ? launch_pass_w(t, pp, stream) : launch_pass(t, rc.fast, pp, stream);

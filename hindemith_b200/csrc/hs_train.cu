@@ -169,6 +169,29 @@ static hs_status launch_table_w(const PassTable &tab, cudaStream_t s) {
     else HS_FAIL(HS_ERR_INVALID_ARG, "recompute pass depth %d above %d", T, kMaxDumpDepth);
 }
 
+// Warps of a table pass's kernel that an SM holds at once (its launch bound is the least it may hold).
+template <int T, int WP>
+static int table_warps_wp(bool fast, bool wide) {
+    static std::atomic<int> held[3][64];
+    const size_t smem = WP * sizeof(float) * (wide ? GeoW<T>::warp_floats : Geo<T>::warp_floats);
+    return wide   ? std::max(held_warps((const void *)hs_table_pass_w_kernel<T, WP>, WP, smem, held[2]), T <= 4 ? 12 : 8)
+           : fast ? std::max(held_warps((const void *)hs_table_pass_kernel<T, true, WP>, WP, smem, held[1]),
+                             T <= 4 ? 16 : T <= 6 ? 12 : 8)
+                  : std::max(held_warps((const void *)hs_table_pass_kernel<T, false, WP>, WP, smem, held[0]),
+                             T <= 4 ? 16 : T <= 6 ? 12 : 8);
+}
+static int table_warps(int T, bool fast, bool wide, bool dump) {
+#define HS_CASE(TT) \
+    case TT: return dump ? table_warps_wp<TT, kBackwardWarps>(fast, wide) : table_warps_wp<TT, kPassWarps>(fast, wide);
+    switch (T) {
+        HS_CASE(1) HS_CASE(2) HS_CASE(3) HS_CASE(4) HS_CASE(5)
+        case 6: return table_warps_wp<6, kPassWarps>(fast, wide);
+        case 7: return table_warps_wp<7, kPassWarps>(fast, wide);
+        default: return table_warps_wp<8, kPassWarps>(fast, wide);
+    }
+#undef HS_CASE
+}
+
 static hs_status launch_table_any(int T, bool fast, const PassTable &tab, cudaStream_t s) {
     if (tab.wide) {
         switch (T) {
@@ -674,17 +697,17 @@ static long pair_pixels(const hs_train_pair *pairs, int n) {
     return px / std::max(n, 1);
 }
 
-// rows per work item for a table launch: about one wave of warps over all pairs.  In the
-// 4-columns-per-lane layout the strips are re-cut and the wave holds the warps the wide
-// kernel keeps resident (12 per SM to depth 4, 8 beyond).
-static void set_segments(PassTable &tab, int T) {
+// rows per work item for a table launch: items for 16 warps per SM over all pairs, but not more
+// than the SMs hold at once.  In the 4-columns-per-lane layout the strips are re-cut and there are
+// items for 12 warps per SM to depth 4, 8 beyond.
+static void set_segments(PassTable &tab, int T, bool fast) {
     if (tab.wide)
         for (int i = 0; i < tab.npairs; ++i)
             tab.pair[i].nstrips = (tab.pair[i].W + strip_cols_wide(T) - 1) / strip_cols_wide(T);
     long rows = 0;
     for (int i = 0; i < tab.npairs; ++i) rows += (long)tab.pair[i].nstrips * tab.pair[i].H;
-    // (the narrow kernel's resident warps: 16 to depth 4, 12 to 6, 8 beyond)
-    const long target = (long)sm_count() * (tab.wide ? (T <= 4 ? 12 : 8) : (T <= 4 ? 16 : T <= 6 ? 12 : 8));
+    const long target = (long)sm_count() * (tab.wide ? (T <= 4 ? 12 : 8) : 16);
+    const long slots = (long)sm_count() * table_warps(T, fast, tab.wide, tab.pair[0].dump != 0);
     int L = (int)std::max(1L, (rows + target - 1) / target);
     L = std::max(L, std::max(8, 2 * T));
     // each image rounds its last segment up: longer segments until the items are one wave
@@ -695,7 +718,7 @@ static void set_segments(PassTable &tab, int T) {
             items += (long)tab.pair[i].nstrips * ((tab.pair[i].H + L - 1) / L);
             more |= L < tab.pair[i].H;
         }
-        if (items <= target || !more) break;
+        if (items <= slots || !more) break;
     }
     tab.item_prefix[0] = 0;
     for (int i = 0; i < tab.npairs; ++i) {
@@ -758,7 +781,7 @@ static hs_status train_forward(const hs_train_pair *pairs, const PairBufs *bufs,
                 p.v_out = q == passes - 1 ? B.ck(b + 1, 1) : B.scr(q & 1, 1);
                 tab.pair[i] = p;
             }
-            set_segments(tab, t);
+            set_segments(tab, t, rc.fast);
             if ((st = launch_table_any(t, rc.fast, tab, s)) != HS_OK) return st;
             done += t;
         }
@@ -893,7 +916,7 @@ static hs_status train_backward(const hs_train_pair *pairs, const PairBufs *bufs
                 p.v_out = p.dump_v[t - 1];
                 tab.pair[i] = p;
             }
-            set_segments(tab, t);
+            set_segments(tab, t, rc.fast);
             hs_status e = launch_table_any(t, rc.fast, tab, ds);
             if (e != HS_OK) return e;
             done += t;

@@ -12,6 +12,7 @@ static int nkernels;
 static char *text;
 static size_t len, cap;
 static int coop_limit = 1 << 30; /* cooperative launches of more blocks are refused */
+static int held = 16; /* warps of any kernel that an SM holds at once */
 static int queries; /* calls that ask for the device or an attribute */
 
 static void record(const char *fmt, ...) {
@@ -33,6 +34,7 @@ void fake_reset(int max_cooperative_blocks) {
     coop_limit = max_cooperative_blocks;
     record("%s", "");
 }
+void fake_hold(int warps) { held = warps; }
 const char *fake_log(void) { return text ? text : ""; }
 int fake_queries(void) { return queries; }
 
@@ -105,9 +107,13 @@ cudaError_t cudaFuncSetAttribute(const void *f, enum cudaFuncAttribute a, int v)
     return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const void *f, int b, size_t s, unsigned fl) {
-    (void)f; (void)b; (void)s; (void)fl;
-    *n = 2;
+    (void)f; (void)s; (void)fl;
+    ++queries;
+    *n = held / (b / 32);
     return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int *n, const void *f, int b, size_t s) {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(n, f, b, s, 0);
 }
 cudaError_t cudaGetSymbolAddress(void **p, const void *sym) { (void)sym; *p = (void *)(uintptr_t)0x7000000000; return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned f) { (void)f; *s = (cudaStream_t)(uintptr_t)1; return cudaSuccess; }

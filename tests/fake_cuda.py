@@ -31,7 +31,9 @@ def _parse(mangled):
 
 
 class FakeCuda:
-    def __init__(self):
+    """held: warps of any kernel that an SM holds at once (the library asks once and keeps it)."""
+
+    def __init__(self, held=16):
         B.build()
         self.dir = tempfile.TemporaryDirectory()
         so = os.path.join(self.dir.name, "libhsflow_fake.so")
@@ -46,6 +48,7 @@ class FakeCuda:
             f = getattr(self.lib, name)
             f.restype, f.argtypes = res, args
         self.lib.fake_log.restype = ctypes.c_char_p
+        self.lib.fake_hold(held)
         self.reset()
 
     def reset(self, max_cooperative_blocks=1 << 30):
@@ -61,12 +64,11 @@ class FakeCuda:
         return out
 
 
-_fake = None
+_fakes = {}
 
 
-def fake_cuda():
-    global _fake
-    if _fake is None:
-        _fake = FakeCuda()
-    _fake.reset()
-    return _fake
+def fake_cuda(held=16):
+    if held not in _fakes:
+        _fakes[held] = FakeCuda(held)
+    _fakes[held].reset()
+    return _fakes[held]

@@ -189,3 +189,46 @@ def test_batch_of_large_pairs_and_small_ones_does_each_once(fake):
     assert [x.first for x in ls if x.kernel == "derivs_kernel"] == at[:1]
     assert [x.first for x in ls if x.kernel == "hs_resident_kernel"] == at[1:2]
     assert [x.first for x in ls if x.kernel == "batch_derivs_kernel"] == at[2:3]
+
+
+# ------------------------------------------------------------------ rows per work item
+
+def pass_items(f, H, W, cfg, T):
+    """Work items of the passes of 2 T sweeps (one warp each)."""
+    ld = pad(W)
+    need = f.lib.hs_sweeps_workspace_bytes(H, W, ld)
+    planes = [P((1 << 36) + k * 256 * MB) for k in range(5)]
+    f.reset()
+    assert f.lib.hs_sweeps(*planes[:3], H, W, ld, 1.0, 2 * T, *planes[3:], P(WS), need, ctypes.byref(cfg), None) == L.HS_OK
+    out = {x.grid * (x.threads // 32) for x in f.launches()}
+    assert len(out) == 1
+    return out.pop()
+
+
+@pytest.mark.parametrize("held", [8, 12, 16, 19, 28])
+@pytest.mark.parametrize("H,W", [(1080, 1920), (1811, 2048), (2160, 3840), (64, 30000)])
+@pytest.mark.parametrize("T", [1, 5, 7])
+@pytest.mark.parametrize("layout", [1, 2])
+def test_passes_fill_the_warps_the_kernel_holds(held, H, W, T, layout):
+    """Items for 16 warps per SM (4 columns per lane: 12, 8 beyond depth 4) where the SMs hold them
+    at once, else as many as they hold in whole strips; a kernel never holds less than its launch
+    bound."""
+    f = fake_cuda(held)
+    bound = (12 if T <= 4 else 8) if layout == 2 else (16 if T <= 4 else 12 if T <= 6 else 8)
+    want = bound if layout == 2 else 16
+    slots = max(held, bound) * 148
+    strips = -(-W // (128 - 2 * ((T + 3) // 4 * 4))) if layout == 2 else -(-W // (64 - 2 * (T + T % 2)))
+    items = pass_items(f, H, W, L.make_config(fast_math=True, sweeps_per_pass=T, layout=layout), T)
+    items -= items % strips  # (the last CTA of four warps may not be full)
+    seg = lambda n: -(-H // max(-(-H // n), 2 * T, 8))
+    full = seg(-(-148 * want // strips))
+    assert items == strips * (full if full * strips <= slots else seg(max(1, slots // strips)))
+
+
+def test_training_passes_fill_the_warps_the_kernel_holds():
+    """Two intervals' recompute passes of 16 x 512^2: 16 warps per SM where they are held."""
+    for held, most in ((16, 16 * 148), (12, 12 * 148)):
+        f = fake_cuda(held)
+        ls = train(f, [(512, 512)] * 16, 20, 10, cfg=L.make_config(fast_math=True, sweeps_per_pass=5), backward=True)
+        items = {x.grid * (x.threads // 32) for x in ls if x.kernel == "hs_table_pass_kernel" and x.args[0] == 5}
+        assert len(items) == 1 and 0.75 * most < items.pop() <= most

@@ -155,9 +155,15 @@ static int pass_warps(int T, bool fast) { return HS_BY_DEPTH(pass_warps_at, T, f
 static int pass_warps_w(int T, bool tm) { return HS_BY_DEPTH(pass_warps_w_at, T, tm); }
 #undef HS_BY_DEPTH
 
+// Depths 2 and 3 hold fewer warps with the ring in tensor memory than without (12 against 15 and 13:
+// registers), so with given segments that leave a small second wave, up to a third, the one-warp
+// CTAs are faster (4096^2 in segments of 64 rows, T = 2 x 8 sweeps 398 us against 458, T = 3 x 12 422
+// against 441; with one wave, or more than that of a second, the ring in tensor memory is: segments
+// of 128 rows 526 -> 393 and 572 -> 431; at T = 1 always).
 template <int T>
 static hs_status launch_one_w(const SweepParams &pp, cudaStream_t stream) {
-    if ((long)pp.H * pp.W < kTmPixels) {
+    const long slots = T == 2 || T == 3 ? (long)sm_count() * pass_warps_w_at<T>(true) : 0;
+    if ((long)pp.H * pp.W < kTmPixels || (pp.nitems > slots && 3L * pp.nitems <= 4 * slots)) {
         static bool attr_set[64] = {};
         return launch_kernel(hs_stream_w_kernel<T>, kPassWarps * GeoW<T>::warp_floats * (int)sizeof(float), attr_set,
                              pp, stream);

@@ -232,3 +232,16 @@ def test_training_passes_fill_the_warps_the_kernel_holds():
         ls = train(f, [(512, 512)] * 16, 20, 10, cfg=L.make_config(fast_math=True, sweeps_per_pass=5), backward=True)
         items = {x.grid * (x.threads // 32) for x in ls if x.kernel == "hs_table_pass_kernel" and x.args[0] == 5}
         assert len(items) == 1 and 0.75 * most < items.pop() <= most
+
+
+@pytest.mark.parametrize("T,rows,kernel", [(2, 0, "hs_stream_tm_kernel"), (2, 64, "hs_stream_w_kernel"), (3, 64, "hs_stream_w_kernel"),
+                                           (2, 128, "hs_stream_tm_kernel"), (2, 32, "hs_stream_tm_kernel"),
+                                           (1, 64, "hs_stream_tm_kernel"), (4, 64, "hs_stream_tm_kernel")])
+def test_large_images_at_small_depths_avoid_a_small_second_wave(T, rows, kernel):
+    f = fake_cuda(12)
+    H = W = 4096
+    need = f.lib.hs_sweeps_workspace_bytes(H, W, W)
+    planes = [P((1 << 36) + k * 256 * MB) for k in range(5)]
+    cfg = L.make_config(fast_math=True, sweeps_per_pass=T, layout=2, rows_per_segment=rows)
+    assert f.lib.hs_sweeps(*planes[:3], H, W, W, 1.0, 2 * T, *planes[3:], P(WS), need, ctypes.byref(cfg), None) == L.HS_OK
+    assert kernels(f.launches()) == {kernel}

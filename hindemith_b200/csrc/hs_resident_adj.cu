@@ -358,6 +358,34 @@ static hs_status launch_resident_adj(const ResAdjTable &tab, cudaStream_t s) {
     return HS_OK;
 }
 
+// When the backward runs here and when in the streaming passes (hs_train.cu): the time of a sweep with
+// its recompute in one launch here, of r rows per warp and mpx Mpx, and in the passes for n images.
+// Both are fits to 752 backwards measured on B200, 64^2 .. 1920x1080, 1 .. 32 images, intervals of 1 ..
+// 32 sweeps, both forms (each 10 % r.m.s.).  By this rule they take 0.757 of the passes' time in the
+// geometric mean, by the faster way each time 0.754, and none takes more than 1.10 of it.
+//   here  : the tile's rows (the exact form divides in its recompute), the states' way through L2 and,
+//           past it, through HBM, and an exchange every kResT sweeps or every interval;
+//   passes: launches below 0.17 Mpx, the planes' traffic above.  An interval of one sweep recomputes
+//           nothing, one of two sweeps takes a pass for its one.
+// Measured, us per sweep here / in the passes, intervals of 10, fast form: 320x240 5.4 / 4.9 (exact
+// 6.6 / 7.0), 2 of 200x192 3.9 / 5.1, 512^2 6.7 / 8.9 (intervals of 1: 8.5 / 5.8), 4 of 512^2 12.0 / 13.2,
+// 16 of 512^2 47.6 / 36.7.
+static double adj_sweep_us(int r, double mpx, bool several, int ckpt_every, bool fast) {
+    static const double rows[2][kAdjMaxR - 1] = {{2.3, 4.4, 6.1, 7.3, 9.0}, {2.6, 4.3, 4.5, 6.0, 7.0}};
+    const double spilled = std::max(0.0, mpx * 16.0 * (ckpt_every - 1) - 120.0);  // MB of states beyond L2
+    return rows[fast][r - 2] + (fast ? 2.7 : 3.5) * mpx + (fast ? 0.0014 : 0.0025) * spilled +
+           (several ? 2.6 / std::min(ckpt_every, kResT) : 0.0);
+}
+static double passes_sweep_us(int n, double mpx, int ckpt_every, bool fast) {
+    const bool small = mpx < 0.17;
+    double us;
+    if (ckpt_every == 1) us = small ? 3.3 + 7.0 * mpx : 4.8 + 3.8 * mpx;
+    else if (ckpt_every == 2) us = 8.0 + 7.3 * mpx;
+    else if (small) us = (ckpt_every == 3 ? 6.5 : ckpt_every == 4 ? 4.2 : fast ? 4.6 : 6.0) + (fast ? 6.0 : 9.0) * mpx;
+    else us = fast ? 7.0 + 5.5 * mpx + std::max(0.0, mpx - 2.0) : 8.2 + 8.0 * mpx + std::max(0.0, mpx - 2.0);
+    return us + 0.15 * (n - 1);
+}
+
 hs_status run_resident_adjoint(const ResidentAdjJob *jobs, int n, int iters, int ckpt_every, size_t plane, int nslots,
                                const ResolvedConfig &rc, cudaStream_t s) {
     std::vector<ResidentJob> sizes(n);
@@ -368,23 +396,22 @@ hs_status run_resident_adjoint(const ResidentAdjJob *jobs, int n, int iters, int
         sizes[i].iters = iters;
         sizes[i].scratch_bytes = jobs[i].scratch_bytes;
     }
-    // A sweep and its recompute take about 1.2 + 1.45 r us per launch here, a third more where the
-    // launch's states outgrow L2, and 7 + 8 us per Mpx in the streaming passes (measured on B200: one
-    // 512^2 image 6.9 against 8.7 us, 2 of 1024^2 two launches of 10.8 against 21.5, 16 of 512^2 four
-    // of 13.4 against 40): a few small images are reversed here, where the streaming passes are
-    // launches; large batches there.
     ResidentCut cut;
-    const double base = 1.2, slope = 1.45;
-    if (!resident_cut(sizes.data(), n, base, slope, kAdjMaxR, cut)) return HS_ERR_UNSUPPORTED;
+    if (!resident_cut(sizes.data(), n, 1.2, 1.45, kAdjMaxR, cut)) return HS_ERR_UNSUPPORTED;
     double here = 0.0, pixels = 0.0;
     for (size_t l = 0; l < cut.end.size(); ++l) {
+        const int r = cut.r[l];
         double px = 0.0;
-        for (int i = l ? cut.end[l - 1] : 0; i < cut.end[l]; ++i) px += (double)jobs[i].H * jobs[i].W;
-        const bool spills = px * 16.0 * (ckpt_every - 1) > 120e6;  // two buffers of k - 1 plane pairs
-        here += (base + slope * cut.r[l]) * (spills ? 1.35 : 1.0);
+        bool several = false;
+        for (int i = l ? cut.end[l - 1] : 0; i < cut.end[l]; ++i) {
+            int ntx, nty;
+            px += 1e-6 * jobs[i].H * jobs[i].W;
+            several |= resident_tiles(jobs[i].H, jobs[i].W, r, &ntx, &nty) > 1;
+        }
+        here += adj_sweep_us(r, px, several, ckpt_every, rc.fast);
         pixels += px;
     }
-    if (here > 7.0 + 8e-6 * pixels) return HS_ERR_UNSUPPORTED;
+    if (here > passes_sweep_us(n, pixels, ckpt_every, rc.fast)) return HS_ERR_UNSUPPORTED;
     for (size_t l = 0; l < cut.end.size(); ++l) {
         const int i0 = l ? cut.end[l - 1] : 0, m = cut.end[l] - i0, r = cut.r[l];
         ResAdjTable tab;

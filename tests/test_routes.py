@@ -245,3 +245,43 @@ def test_large_images_at_small_depths_avoid_a_small_second_wave(T, rows, kernel)
     cfg = L.make_config(fast_math=True, sweeps_per_pass=T, layout=2, rows_per_segment=rows)
     assert f.lib.hs_sweeps(*planes[:3], H, W, W, 1.0, 2 * T, *planes[3:], P(WS), need, ctypes.byref(cfg), None) == L.HS_OK
     assert kernels(f.launches()) == {kernel}
+
+
+# ------------------------------------------------------------------ the backward's two ways
+
+def single(fake, H, W, iters, ckpt, fast):
+    """Kernels of hs_backward for one pair."""
+    cfg = L.make_config(fast_math=fast)
+    ld = pad(W)
+    need = fake.lib.hs_backward_workspace_bytes(H, W, ld, ckpt)
+    a = [P((1 << 36) + k * 64 * MB) for k in range(8)]
+    fake.reset()
+    assert fake.lib.hs_backward(a[0], H, W, ld, a[1], iters, ckpt, a[2], a[3], a[4], a[5], a[6], a[7], P(WS), need,
+                                ctypes.byref(cfg), None) == L.HS_OK
+    return fake.launches()
+
+
+# measured on B200, us: the passes against the chip (in brackets the one not taken)
+@pytest.mark.parametrize("shapes,iters,ckpt,fast,resident", [
+    ([(240, 320)], 200, 10, True, False),         # 948 (1065)
+    ([(240, 320)], 200, 10, False, True),         # (1368) 1310
+    ([(64, 64)] * 2, 200, 10, True, False),       # 4.98 (5.68) a sweep
+    ([(128, 128)] * 2, 200, 10, True, False),     # 959 (1101)
+    ([(512, 512)] * 8, 50, 5, True, False),       # 1066 (1275)
+    ([(512, 512)] * 16, 50, 5, True, False),      # 2037 (2529)
+    ([(512, 512)] * 16, 50, 5, False, False),     # 2564 (3042)
+    ([(600, 800)], 100, 1, True, False),          # 603 (977): no recompute in the passes
+    ([(512, 512)] * 4, 100, 1, False, False),     # 809 (1837)
+    ([(437, 613)], 100, 10, False, True),         # (1044) 860
+    ([(256, 256)] * 4, 200, 10, True, True),      # (1885) 760
+    ([(512, 512)] * 2, 200, 10, True, True),      # (2260) 1094
+    ([(512, 512)] * 4, 100, 16, False, True),     # (1996) 1449
+    ([(128, 128)] * 32, 200, 10, True, True),     # (2746) 1562
+])
+def test_backward_takes_the_faster_way(fake, shapes, iters, ckpt, fast, resident):
+    if len(shapes) == 1:
+        ls = single(fake, *shapes[0], iters, ckpt, fast)
+    else:
+        ls = train(fake, shapes, iters, ckpt, cfg=L.make_config(fast_math=fast), backward=True)
+    assert ("hs_resident_adj_kernel" in kernels(ls)) == resident
+    assert ("hs_adjoint_pass_kernel" in kernels(ls)) == (not resident)

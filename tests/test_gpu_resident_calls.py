@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from conftest import assert_bitexact
+from resident_cases import CKPT, GROUPS, ITERS, SINGLE
 from hindemith_b200 import _lib as L
 from hindemith_b200 import device as D
 
@@ -44,6 +45,11 @@ def test_forward_writing_inside_its_images_memory(cuda, fast, rows):
 
 # ------------------------------------------------------------------ the backward's sums
 
+def poisoned(n):
+    """n bytes of NaN."""
+    return torch.full((n,), 255, dtype=torch.uint8, device="cuda")
+
+
 class SinglePair:
     """hs_forward_train and hs_backward on buffers of the test's own, whose parts it reads."""
 
@@ -55,11 +61,12 @@ class SinglePair:
         self.I0, self.I1 = images((H, W), 2, seed)
         self.stride = (H * self.ld * 4 + 255) // 256 * 256
         self.alpha = torch.tensor([0.9], device="cuda")
-        u, v = images((H, W), 2, 0)
+        self.flow = images((H, W), 2, 0)
+        u, v = self.flow
         nd = self.lib.hs_derivs_bytes(H, W, self.ld)
         nc = self.lib.hs_checkpoint_bytes(H, W, self.ld, iters, ckpt)
         nw = self.lib.hs_forward_train_workspace_bytes(H, W, self.ld)
-        self.derivs, self.planes, ws = (torch.zeros(n, dtype=torch.uint8, device="cuda") for n in (nd, nc, nw))
+        self.derivs, self.planes, ws = (poisoned(n) for n in (nd, nc, nw))
         L.check(self.lib.hs_forward_train(D.ptr(self.I0), D.ptr(self.I1), H, W, self.ld, D.ptr(self.alpha), iters, ckpt,
                                           D.ptr(u), D.ptr(v), D.ptr(self.derivs), D.ptr(self.planes), D.ptr(ws), nw,
                                           self.cfg, D.stream_handle()), "hs_forward_train")
@@ -68,23 +75,23 @@ class SinglePair:
         b = buf[k * self.stride:k * self.stride + self.H * self.ld * 4].view(torch.float32)
         return b.view(self.H, self.ld)[:, :self.W]
 
-    def backward(self, first, intervals, iters, ckpt, lu, lv):
-        """The sweeps from checkpoint plane `first` on; (accumulators, lambda parked before the first
-        interval)."""
+    def backward(self, first, iters, ckpt, lu, lv, cfg=None):
+        """The sweeps from checkpoint plane `first` on: (accumulators, lambda parked before the first
+        interval, gradients)."""
         need = self.lib.hs_backward_workspace_bytes(self.H, self.W, self.ld, ckpt)
-        ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+        ws = poisoned(need)
         out = images((self.H, self.W), 2, 0)
         da = torch.zeros(1, device="cuda")
         at = self.ct.c_void_p(self.planes.data_ptr() + 2 * first * self.stride)
         L.check(self.lib.hs_backward(D.ptr(self.derivs), self.H, self.W, self.ld, D.ptr(self.alpha), iters, ckpt, at, D.ptr(lu),
-                                     D.ptr(lv), D.ptr(out[0]), D.ptr(out[1]), D.ptr(da), D.ptr(ws), need, self.cfg,
-                                     D.stream_handle()), "hs_backward")
+                                     D.ptr(lv), D.ptr(out[0]), D.ptr(out[1]), D.ptr(da), D.ptr(ws), need,
+                                     self.cfg if cfg is None else self.ct.byref(cfg), D.stream_handle()), "hs_backward")
         lam = 4 * (ckpt - 1)
         return ([self.plane(ws, lam + 4 + i).clone() for i in range(3)],
-                [D.as_plane(self.plane(ws, lam + i).clone()) for i in range(2)])
+                [D.as_plane(self.plane(ws, lam + i).clone()) for i in range(2)], [*out, da])
 
 
-@pytest.mark.parametrize("ckpt", [1, 100])
+@pytest.mark.parametrize("ckpt", [1, 10, 100])
 def test_backward_sums_no_further_off_than_the_passes_order(cuda, ckpt):
     """dIx, dIy, dIt over 100 sweeps: the same terms as 25 backwards of 4 sweeps each.  Against
     these added in 64 bits, the sums of one call are no further off than these added in 32 bits one
@@ -94,18 +101,57 @@ def test_backward_sums_no_further_off_than_the_passes_order(cuda, ckpt):
     lam = images((H, W), 2, 7)
     four = SinglePair(H, W, n, 4, cfg, 3)
     one = SinglePair(H, W, n, ckpt, cfg, 3)
-    got, _ = one.backward(0, n // ckpt, n, ckpt, *lam)
+    got = one.backward(0, n, ckpt, *lam)[0]
     sum64, sum32 = [0.0] * 3, None
     l = lam
     for c in range(n // 4 - 1, -1, -1):
-        acc, _ = four.backward(c, 1, 4, 4, *l)
+        acc = four.backward(c, 4, 4, *l)[0]
         sum64 = [s + a.double() for s, a in zip(sum64, acc)]
         sum32 = [s + a for s, a in zip(sum32, acc)] if sum32 else acc
         if c:
-            l = four.backward(c - 1, 2, 8, 4, *l)[1]
+            l = four.backward(c - 1, 8, 4, *l)[1]
     for k in range(3):
         off = [float((s.double() - sum64[k]).norm()) for s in (got[k], sum32[k])]
         assert off[0] <= 1.1 * off[1], (k, off)
+
+
+@pytest.mark.parametrize("fast", [True, False])
+@pytest.mark.parametrize("H,W,rows", SINGLE)
+def test_single_pair_at_every_tile_height(cuda, H, W, rows, fast):
+    """Forward and backward of one pair on the chip and in the passes, in all four combinations, on
+    buffers full of NaN: the same flow bit for bit, gradients within 1e-5 of their norm."""
+    auto, passes = L.make_config(fast_math=fast), L.make_config(fast_math=fast, sweeps_per_pass=4)
+    lam = images((H, W), 2, 7)
+    pairs = [SinglePair(H, W, ITERS, CKPT, cfg, 3) for cfg in (passes, auto)]
+    for a, b in zip(pairs[0].flow, pairs[1].flow):
+        equal(b, a, "flow")
+    ref = pairs[0].backward(0, ITERS, CKPT, *lam, cfg=passes)[2]
+    for p, cfg in ((pairs[0], auto), (pairs[1], passes), (pairs[1], auto)):
+        for g, r in zip(p.backward(0, ITERS, CKPT, *lam, cfg=cfg)[2], ref):
+            assert (g - r).norm() <= 1e-5 * r.norm()
+
+
+@pytest.mark.parametrize("fast", [True, False])
+@pytest.mark.parametrize("shapes", [g[0] for g in GROUPS])
+def test_training_batches_of_several_launches(cuda, shapes, fast):
+    from hindemith_b200.autograd import horn_schunck_batch
+
+    ims = [images(s, 2, 20 + i) for i, s in enumerate(shapes)]
+    lam = [images(s, 2, 80 + i) for i, s in enumerate(shapes)]
+
+    def run(cfg):
+        nan = torch.full((1 << 28,), float("nan"), device="cuda")  # what the call's buffers hold
+        del nan
+        a = torch.tensor(0.8, device="cuda", requires_grad=True)
+        xs = [tuple(t.clone().requires_grad_(True) for t in p) for p in ims]
+        outs = [t for o in horn_schunck_batch(xs, a, ITERS, CKPT, cfg) for t in o]
+        return outs, torch.autograd.grad(outs, [t for x in xs for t in x] + [a], [t for p in lam for t in p])
+
+    (f0, g0), (f1, g1) = run(L.make_config(fast_math=fast)), run(L.make_config(fast_math=fast, sweeps_per_pass=4))
+    for a, b in zip(f0, f1):
+        equal(a, b, "flow")
+    for a, b in zip(g0, g1):
+        assert (a - b).norm() <= 1e-5 * b.norm()
 
 
 # ------------------------------------------------------------------ the batched call's default

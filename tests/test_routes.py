@@ -285,3 +285,20 @@ def test_backward_takes_the_faster_way(fake, shapes, iters, ckpt, fast, resident
         ls = train(fake, shapes, iters, ckpt, cfg=L.make_config(fast_math=fast), backward=True)
     assert ("hs_resident_adj_kernel" in kernels(ls)) == resident
     assert ("hs_adjoint_pass_kernel" in kernels(ls)) == (not resident)
+
+
+# ------------------------------------------------------------------ what the GPU tests of training reach
+
+@pytest.mark.parametrize("fast", [True, False])
+def test_training_cases_take_their_tile_heights(fake, fast):
+    from resident_cases import CKPT, GROUPS, ITERS, SINGLE
+
+    cfg = L.make_config(fast_math=fast)
+    for H, W, rows in SINGLE:
+        assert [x.args for x in single(fake, H, W, ITERS, CKPT, fast) if x.kernel == "hs_resident_adj_kernel"] == [(fast, rows)]
+    assert {rows for _, _, rows in SINGLE} == {2, 3, 4, 5, 6}
+    for shapes, forward_rows, backward_rows in GROUPS:
+        for name, back, rows in (("hs_resident_kernel", False, forward_rows), ("hs_resident_adj_kernel", True, backward_rows)):
+            fake.reset()
+            ls = train(fake, shapes, ITERS, CKPT, cfg=cfg, backward=back)
+            assert [x.args[-1] for x in ls if x.kernel == name] == rows

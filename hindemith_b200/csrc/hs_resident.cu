@@ -136,13 +136,12 @@ __global__ void __launch_bounds__(NW * 32, 1) hs_resident_kernel(const __grid_co
         if (b + 1 == p.nblocks) break;
         if (p.ntx * p.nty == 1) continue;  // no neighbours
 
-        if (!res_exchange<NW, R, false>(t, g, cu, out, in, src, p.box, (unsigned)(b + 1), &stop, tab.abort_flag,
-                                        tab.status)) {
+        if (!res_exchange<NW, R, false>(t, g, cu, out, in, src, p.box, (unsigned)(b + 1), &stop, tab.wait)) {
             ok = false;
             break;
         }
     }
-    if (p.nblocks > 1) ok = ok && *(volatile unsigned *)tab.abort_flag == 0u;
+    if (p.nblocks > 1) ok = ok && *(volatile unsigned *)tab.wait.abort_flag == 0u;
     if (!ok) {
         const float2 nan2 = f2(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
 #pragma unroll
@@ -229,14 +228,14 @@ __global__ void __launch_bounds__(256) res_clear_kernel(const __grid_constant__ 
     while (image + 1 < tab.n && tab.first[image + 1] <= (int)blockIdx.x) ++image;
     const ResImage &p = tab.img[image];
     const int tiles = p.ntx * p.nty, tile = blockIdx.x - tab.first[image];
-    if (blockIdx.x == 0 && threadIdx.x == 0) *tab.abort_flag = 0u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *tab.wait.abort_flag = 0u;
     if (tiles == 1) return;
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int h = 0; h < 2; ++h)
         for (int i = threadIdx.x; i < msgs; i += blockDim.x) p.box[(size_t)(h * tiles + tile) * msgs + i] = z;
 }
 
-// Launches the table (img, n, ckpt_* and abort_flag filled in; every image tiled for r rows per
+// Launches the table (img, n, ckpt_* and wait filled in; every image tiled for r rows per
 // warp).  An image of several tiles has at least one exchange, so that no tile writes its result
 // before its neighbours have read their inputs; an image of a single tile needs none.
 static hs_status launch_table(ResidentTable &tab, int r, bool zero_start, const ResolvedConfig &rc, cudaStream_t s) {
@@ -284,7 +283,8 @@ hs_status run_resident(const float *I0, const float *I1, const float *Ix, const 
     p.ntx = pl.ntx; p.nty = pl.nty;
     p.iters = iters;
     if (pl.box_bytes)
-        tab.abort_flag = reinterpret_cast<unsigned *>(reinterpret_cast<char *>(scratch) + pl.box_bytes - 256);
+        tab.wait.abort_flag = reinterpret_cast<unsigned *>(reinterpret_cast<char *>(scratch) + pl.box_bytes - 256);
+    tab.wait.polls = kResPolls;
     return launch_table(tab, pl.r, zero_start, rc, s);
 }
 
@@ -344,7 +344,7 @@ bool resident_fits(int H, int W, int iters, size_t scratch_bytes) {
 }
 
 hs_status run_resident_jobs(const ResidentJob *jobs, int n, int ckpt_every, size_t ckpt_plane, int *status,
-                            const ResolvedConfig &rc, cudaStream_t s, int *launched) {
+                            const ResolvedConfig &rc, cudaStream_t s, int *launched, int polls) {
     *launched = 0;
     for (int i = 0; i < n; ++i)
         if (jobs[i].iters < 2) return HS_ERR_UNSUPPORTED;
@@ -358,7 +358,8 @@ hs_status run_resident_jobs(const ResidentJob *jobs, int n, int ckpt_every, size
         tab.n = m;
         tab.ckpt_every = ckpt_every;
         tab.ckpt_plane = ckpt_plane;
-        tab.status = status;
+        tab.wait.status = status;
+        tab.wait.polls = polls;
         for (int i = 0; i < m; ++i) {
             const ResidentJob &d = jobs[i0 + i];
             ResImage &p = tab.img[i];
@@ -373,7 +374,7 @@ hs_status run_resident_jobs(const ResidentJob *jobs, int n, int ckpt_every, size
             p.iters = d.iters;
             const int tiles = resident_tiles(d.H, d.W, r, &p.ntx, &p.nty);
             if (tiles > 1)
-                tab.abort_flag = reinterpret_cast<unsigned *>(d.scratch + resident_box_bytes(tiles, r) - 256);
+                tab.wait.abort_flag = reinterpret_cast<unsigned *>(d.scratch + resident_box_bytes(tiles, r) - 256);
         }
         const hs_status st = launch_table(tab, r, true, rc, s);
         if (st != HS_OK) return st;
@@ -383,3 +384,13 @@ hs_status run_resident_jobs(const ResidentJob *jobs, int n, int ckpt_every, size
 }
 
 }  // namespace hs
+
+using namespace hs;
+
+extern "C" hs_status hs_wait_status(int *device_status, void *stream) {
+    clear_error();
+    if (!device_status) HS_FAIL(HS_ERR_INVALID_ARG, "device_status is NULL");
+    wait_status_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(device_status, 1);
+    HS_LAUNCH_CHECK("wait_status_kernel");
+    return resident_adjoint_wait_status(device_status, (cudaStream_t)stream);
+}

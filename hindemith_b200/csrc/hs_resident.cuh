@@ -49,6 +49,23 @@ constexpr int kResChunks = kResCols / 4 - 2;  // 4-column chunks of a tile's own
 
 constexpr int kMaxResImages = 32;  // images of one launch
 
+// What a launch's waits share.
+struct ResWait {
+    unsigned *abort_flag;  // raised by a wait that ran out
+    int *status;           // if set: HS_ERR_TIMEOUT goes here then
+    int polls;             // of one message, at most
+};
+
+// Set to HS_ERR_TIMEOUT, too, when a wait of any launch runs out, until hs_wait_status reads it.  (One
+// word per translation unit: a device pointer to a single one would take host work in every call.)
+static __device__ int g_wait_status;
+
+// *out: the word, which is cleared, or what is there already if it is set.
+static __global__ void wait_status_kernel(int *out, int first) {
+    const int word = atomicExch(&g_wait_status, 0);
+    if (first || word) *out = word;
+}
+
 struct ResImage {
     const float *I0, *I1;        // if set: the images; the kernel forms the derivatives itself
     float *Ix, *Iy, *It;         // else the derivative planes; with the images: where to keep them, or null
@@ -67,8 +84,7 @@ struct ResidentTable {
     ResImage img[kMaxResImages];
     int first[kMaxResImages + 1];  // tiles of the images before image i
     int n;
-    unsigned *abort_flag;        // raised by a wait that ran out
-    int *status;                 // if set: HS_ERR_TIMEOUT goes here then
+    ResWait wait;
     size_t ckpt_plane;           // floats between checkpoint planes
     int ckpt_every;
     float we, wc;
@@ -379,10 +395,11 @@ constexpr int res_tmem_cols() {
     return words <= 32 ? 32 : words <= 64 ? 64 : words <= 128 ? 128 : words <= 256 ? 256 : 512;
 }
 
-// Polls of one message, at most: a few seconds.  A wait can only run out if a neighbour's CTA
-// has stopped (all CTAs of the cooperative launch are resident together); the tile then raises
-// the abort flag, stops waiting, and the tiles that see the flag write NaN as their result.
-constexpr int kResPolls = 1 << 22;
+// A wait (of kResPolls polls, hs_stream.cuh) can only run out if a neighbour's CTA has stopped: the
+// CTAs of a cooperative launch are resident together, and start together (measured on B200: with
+// another kernel on five SMs none of 148 CTAs started before the five were free, then all within a
+// microsecond).  The tile then raises the abort flag, sets the status words and stops waiting, and
+// the tiles that see the flag write NaN as their result.
 
 // One 128-bit access of a message (single-copy atomic).
 __device__ __forceinline__ void msg_store(float4 *p, float a, float b, float c, unsigned e) {
@@ -512,7 +529,7 @@ __device__ __forceinline__ void res_sources(const ResTile &g, int *src, float *i
 template <int NW, int R, bool FENCE>
 __device__ __forceinline__ bool res_exchange(const ResLane &t, const ResTile &g, float2 (&cu)[R][2][2], float *out,
                                              float *in, const int *src, float4 *box, unsigned e, int *stop,
-                                             unsigned *abort_flag, int *status) {
+                                             const ResWait &w) {
     using S = ResSmem<NW, R>;
     // (uniform in the warp) rows of the ring, and rows of the halo, among the warp's
     const int row_end = t.row0 + R;
@@ -561,10 +578,11 @@ __device__ __forceinline__ bool res_exchange(const ResLane &t, const ResTile &g,
 #pragma unroll
         for (int i = 0; i < kPer; ++i) all = all && tag[i] == e;
         if (all) break;
-        if (++polls > kResPolls ||
-            ((polls & 1023) == 0 && (*(volatile int *)stop || *(volatile unsigned *)abort_flag))) {
-            atomicExch(abort_flag, 1u);
-            if (status) atomicCAS(status, 0, (int)HS_ERR_TIMEOUT);
+        if (++polls > w.polls ||
+            ((polls & 1023) == 0 && (*(volatile int *)stop || *(volatile unsigned *)w.abort_flag))) {
+            atomicExch(w.abort_flag, 1u);
+            if (w.status) atomicCAS(w.status, 0, (int)HS_ERR_TIMEOUT);
+            atomicCAS(&g_wait_status, 0, (int)HS_ERR_TIMEOUT);
             *(volatile int *)stop = 1;
             break;
         }

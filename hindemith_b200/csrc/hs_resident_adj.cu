@@ -47,7 +47,7 @@ struct ResAdjTable {
     ResAdjImage img[kMaxResImages];
     int first[kMaxResImages + 1];
     int n;
-    unsigned *abort_flag;
+    ResWait wait;
     size_t plane;                // floats between planes
     int ckpt_every, iters, nslots;
     int chain;                   // sweeps whose terms are summed before they join the planes
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 1) hs_resident_adj_kernel(cons
             load(p.ckpt + (size_t)(2 * b) * pl, p.ckpt + (size_t)(2 * b + 1) * pl, false);
             for (int s = 1; s < nsw; ++s) {
                 if (s > 1 && (s - 1) % kResT == 0 && tiles > 1)
-                    if (!(ok = res_exchange<NW, R, false>(t, g, cu, out, in, src, p.box, ++e, &stop, tab.abort_flag, nullptr)))
+                    if (!(ok = res_exchange<NW, R, false>(t, g, cu, out, in, src, p.box, ++e, &stop, tab.wait)))
                         break;
                 res_run<FAST, NW, R>(t, g, cu, pub, half, 1, tab.we, tab.wc);
                 half ^= 1;
@@ -261,8 +261,8 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 1) hs_resident_adj_kernel(cons
             }
             --left;
             if ((nsw - m) % kResT == 0 && tiles > 1) {
-                ok = m == nsw ? res_exchange<NW, R, true>(t, g, cu, out, in, src, p.box, ++e, &stop, tab.abort_flag, nullptr)
-                              : res_exchange<NW, R, false>(t, g, cu, out, in, src, p.box, ++e, &stop, tab.abort_flag, nullptr);
+                ok = m == nsw ? res_exchange<NW, R, true>(t, g, cu, out, in, src, p.box, ++e, &stop, tab.wait)
+                              : res_exchange<NW, R, false>(t, g, cu, out, in, src, p.box, ++e, &stop, tab.wait);
                 if (!ok) break;
             }
             float2 a2[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 1) hs_resident_adj_kernel(cons
         if (b > 0) res_store_own<R>(t, g, cu, p.park, p.park + pl);
     }
     __syncthreads();
-    if (tiles > 1) ok = ok && stop == 0 && *(volatile unsigned *)tab.abort_flag == 0u;
+    if (tiles > 1) ok = ok && stop == 0 && *(volatile unsigned *)tab.wait.abort_flag == 0u;
     if (!ok) {  // a wait ran out: NaN gradients
         const float nanf_ = __int_as_float(0x7fc00000);
         for (int r = 0; r < R; ++r) {
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(256) res_adj_clear_kernel(const __grid_constan
     while (image + 1 < tab.n && tab.first[image + 1] <= (int)blockIdx.x) ++image;
     const ResAdjImage &p = tab.img[image];
     const int tiles = p.ntx * p.nty, tile = blockIdx.x - tab.first[image];
-    if (blockIdx.x == 0 && threadIdx.x == 0) *tab.abort_flag = 0u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *tab.wait.abort_flag = 0u;
     if (tiles == 1) return;
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int h = 0; h < 2; ++h)
@@ -358,6 +358,12 @@ static hs_status launch_resident_adj(const ResAdjTable &tab, cudaStream_t s) {
     return HS_OK;
 }
 
+hs_status resident_adjoint_wait_status(int *device_status, cudaStream_t s) {
+    wait_status_kernel<<<1, 1, 0, s>>>(device_status, 0);
+    HS_LAUNCH_CHECK("wait_status_kernel");
+    return HS_OK;
+}
+
 // When the backward runs here and when in the streaming passes (hs_train.cu): the time of a sweep with
 // its recompute in one launch here, of r rows per warp and mpx Mpx, and in the passes for n images.
 // Both are fits to 752 backwards measured on B200, 64^2 .. 1920x1080, 1 .. 32 images, intervals of 1 ..
@@ -387,7 +393,7 @@ static double passes_sweep_us(int n, double mpx, int ckpt_every, bool fast) {
 }
 
 hs_status run_resident_adjoint(const ResidentAdjJob *jobs, int n, int iters, int ckpt_every, size_t plane, int nslots,
-                               const ResolvedConfig &rc, cudaStream_t s) {
+                               const ResolvedConfig &rc, cudaStream_t s, int polls) {
     std::vector<ResidentJob> sizes(n);
     for (int i = 0; i < n; ++i) {
         memset(&sizes[i], 0, sizeof(ResidentJob));
@@ -417,6 +423,7 @@ hs_status run_resident_adjoint(const ResidentAdjJob *jobs, int n, int iters, int
         ResAdjTable tab;
         memset(&tab, 0, sizeof(tab));
         tab.n = m;
+        tab.wait.polls = polls;
         tab.plane = plane;
         tab.ckpt_every = ckpt_every;
         tab.iters = iters;
@@ -443,7 +450,7 @@ hs_status run_resident_adjoint(const ResidentAdjJob *jobs, int n, int iters, int
             tab.first[i + 1] = tab.first[i] + tiles;
             if (tiles > 1) {
                 several = true;
-                tab.abort_flag = reinterpret_cast<unsigned *>(d.scratch + resident_box_bytes(tiles, r) - 256);
+                tab.wait.abort_flag = reinterpret_cast<unsigned *>(d.scratch + resident_box_bytes(tiles, r) - 256);
             }
             if (tiles > nslots) HS_FAIL(HS_ERR_INVALID_ARG, "internal: %d tiles, %d slots", tiles, nslots);
         }

@@ -425,6 +425,10 @@ hs_status run_passes_dev(const float *Ix, const float *Iy, const float *It, int 
                          float alpha2, const float *alpha_dev, int iters, float *u0, float *v0,
                          float *u1, float *v1, const ResolvedConfig &rc, cudaStream_t stream);
 
+// Polls of one message of a resident launch, at most: a few seconds.
+constexpr int kResPolls = 1 << 22;
+// hs_wait_status's share of hs_resident_adj.cu: *device_status is overwritten if one of its waits ran out.
+hs_status resident_adjoint_wait_status(int *device_status, cudaStream_t s);
 // The resident form (hs_resident.cu): the tiling of an image that fits the chip.
 struct ResidentPlan {
     int r;             // rows per warp
@@ -446,7 +450,7 @@ bool resident_fits(int H, int W, int iters, size_t scratch_bytes);
 // The resident form for many images, each with its own size and sweeps (>= 2), in launches of as
 // many as fit the chip at once; the flow goes to u, v.  Training: derivatives into Ix, Iy, It (may
 // be null), the state after every ckpt_every sweeps into the checkpoint planes (ckpt_plane floats
-// apart; u then v).  status, if set, receives HS_ERR_TIMEOUT when a wait runs out.
+// apart; u then v).  status, if set, receives HS_ERR_TIMEOUT when a wait runs out (of `polls` polls).
 // *launched: the jobs, the first so many, whose launches were made.  HS_ERR_UNSUPPORTED when an
 // image does not fit, or the SMs at hand hold fewer tiles than the device: the caller runs the
 // jobs that were not launched in another way, and those only (a flow may have taken the place of
@@ -461,7 +465,7 @@ struct ResidentJob {
     int H, W, ld, iters;
 };
 hs_status run_resident_jobs(const ResidentJob *jobs, int n, int ckpt_every, size_t ckpt_plane, int *status,
-                            const ResolvedConfig &rc, cudaStream_t s, int *launched);
+                            const ResolvedConfig &rc, cudaStream_t s, int *launched, int polls = kResPolls);
 // The backward of run_resident_jobs' training form (hs_resident_adj.cu): the accumulators dIx, dIy,
 // dIt and the tiles' shares of dL/dalpha^2 (nslots per image).  HS_ERR_UNSUPPORTED as there, or when
 // the streaming passes are the faster ones.
@@ -475,7 +479,7 @@ struct ResidentAdjJob {
     int H, W, ld;
 };
 hs_status run_resident_adjoint(const ResidentAdjJob *jobs, int n, int iters, int ckpt_every, size_t plane, int nslots,
-                               const ResolvedConfig &rc, cudaStream_t s);
+                               const ResolvedConfig &rc, cudaStream_t s, int polls = kResPolls);
 // How jobs, in their order, are cut into launches: launch k holds jobs end[k-1] .. end[k]-1 with
 // r[k] <= max_r rows per warp; a sweep of a launch takes base + slope * r us.
 struct ResidentCut {

@@ -733,7 +733,7 @@ static void set_segments(PassTable &tab, int T, bool fast) {
 // first pass reads checkpoint b and its last pass writes checkpoint b + 1.  The final state
 // (checkpoint nb) is copied to the pairs' u, v.
 static hs_status train_forward(const hs_train_pair *pairs, const PairBufs *bufs, int n, int iters,
-                               int ckpt_every, const ResolvedConfig &rc, cudaStream_t s) {
+                               int ckpt_every, const ResolvedConfig &rc, cudaStream_t s, int polls = kResPolls) {
     hs_status st;
     // Images that fit the chip run there for all sweeps (hs_resident.cuh), in groups of as many
     // as fit at once: one launch instead of one per pass, and no state traffic but the
@@ -747,7 +747,8 @@ static hs_status train_forward(const hs_train_pair *pairs, const PairBufs *bufs,
                        4 * B.pb, d.alpha, 0.f, d.H, d.W, d.ld, iters};
         }
         int launched = 0;
-        st = run_resident_jobs(jobs.data(), n, ckpt_every, bufs[0].pb / sizeof(float), nullptr, rc, s, &launched);
+        st = run_resident_jobs(jobs.data(), n, ckpt_every, bufs[0].pb / sizeof(float), nullptr, rc, s, &launched,
+                               polls);
         if (st != HS_ERR_UNSUPPORTED) return st;
         pairs += launched;
         bufs += launched;
@@ -860,7 +861,7 @@ static hs_status train_finish(const hs_train_pair *pairs, const PairBufs *bufs, 
 // stream capture, or more than 64 devices) the same work runs in order on one stream.
 static hs_status train_backward(const hs_train_pair *pairs, const PairBufs *bufs, int n, int iters,
                                 int ckpt_every, int nslots, const ResolvedConfig &rc,
-                                cudaStream_t s) {
+                                cudaStream_t s, int polls = kResPolls) {
     hs_status st;
     // Images that fit the chip are reversed there (hs_resident_adj.cu).  The exchange scratch is
     // the forward's ping-pong buffers, or lambda's second buffer in the single-pair call.
@@ -874,7 +875,7 @@ static hs_status train_backward(const hs_train_pair *pairs, const PairBufs *bufs
                        B.scratch ? B.scratch : reinterpret_cast<char *>(B.lamb(1, 0)),
                        (B.scratch ? 4 : 2) * B.pb, d.alpha, d.H, d.W, d.ld};
         }
-        st = run_resident_adjoint(jobs.data(), n, iters, ckpt_every, bufs[0].pb / sizeof(float), nslots, rc, s);
+        st = run_resident_adjoint(jobs.data(), n, iters, ckpt_every, bufs[0].pb / sizeof(float), nslots, rc, s, polls);
         if (st == HS_OK) return train_finish(pairs, bufs, n, nslots, s);
         if (st != HS_ERR_UNSUPPORTED) return st;
     }
@@ -1108,6 +1109,33 @@ hs_status hs_backward_batched(const hs_train_pair *pairs, int n, int iters, int 
     std::vector<PairBufs> bufs(n);
     for (int i = 0; i < n; ++i) bufs[i] = bufs_in_workspace(reinterpret_cast<char *>(workspace), L, i);
     return train_backward(pairs, bufs.data(), n, iters, ckpt_every, L.nslots, rc, (cudaStream_t)stream);
+}
+
+hs_status hs_selftest_resident_wait(const hs_train_pair *pairs, int n, int iters, int ckpt_every, void *workspace,
+                                    size_t workspace_bytes, const hs_config *cfg, int max_polls, void *stream) {
+    clear_error();
+    TrainLayout L;
+    hs_status st = train_layout(pairs, n, iters, ckpt_every, L);
+    if (st != HS_OK) return st;
+    ResolvedConfig rc;
+    if ((st = resolve_config(cfg, &rc)) != HS_OK) return st;
+    if (max_polls < 0 || max_polls > kResPolls)
+        HS_FAIL(HS_ERR_INVALID_ARG, "max_polls=%d outside 0..%d", max_polls, kResPolls);
+    if (!workspace || workspace_bytes < L.total)
+        HS_FAIL(HS_ERR_WORKSPACE, "workspace %zu bytes < required %zu", workspace_bytes, L.total);
+    if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
+        HS_FAIL(HS_ERR_ALIGNMENT, "workspace is not 256-byte aligned");
+    for (int i = 0; i < n; ++i) {
+        const void *pl[8] = {pairs[i].I0, pairs[i].I1, pairs[i].u, pairs[i].v, pairs[i].dLdu, pairs[i].dLdv, pairs[i].dI0, pairs[i].dI1};
+        for (int q = 0; q < 8; ++q)
+            if ((st = check_plane(pl[q], "plane")) != HS_OK) return st;
+        if (!pairs[i].alpha || !pairs[i].dalpha) HS_FAIL(HS_ERR_INVALID_ARG, "pair %d: alpha / dalpha (device) NULL", i);
+    }
+    std::vector<PairBufs> bufs(n);
+    for (int i = 0; i < n; ++i) bufs[i] = bufs_in_workspace(reinterpret_cast<char *>(workspace), L, i);
+    cudaStream_t s = (cudaStream_t)stream;
+    if ((st = train_forward(pairs, bufs.data(), n, iters, ckpt_every, rc, s, max_polls)) != HS_OK) return st;
+    return train_backward(pairs, bufs.data(), n, iters, ckpt_every, L.nslots, rc, s, max_polls);
 }
 
 // ---- the single-pair form: the same passes on caller-held derivative and checkpoint

@@ -134,6 +134,16 @@ def release_workspaces() -> None:
 # ------------------------------------------------------------------ operations
 
 
+def check_waits(device=None) -> None:
+    """Synchronise the current stream and raise if a bounded device-side wait of an earlier call has
+    run out (its flow or gradients then hold NaN) since the last check."""
+    status = torch.zeros(1, dtype=torch.int32, device=device or "cuda")
+    with torch.cuda.device(status.device):
+        L.check(L.lib().hs_wait_status(ptr(status), stream_handle()), "hs_wait_status")
+    if int(status.item()) != L.HS_OK:
+        raise L.HSError(int(status.item()), "hs_wait_status", "a device-side wait gave up")
+
+
 @on_stream
 def stencil2d(weights, offx, offy, x: torch.Tensor, out: Optional[torch.Tensor] = None,
               stream=None) -> torch.Tensor:

@@ -105,6 +105,20 @@ HS_API hs_status hs_array2d_copy(const float *b, float *a, int H, int W, int ld,
 
 /* ---- Horn-Schunck ----------------------------------------------------------- */
 
+/* Images held on the chip (hs_config.sweeps_per_pass, and the calls below): the tiles exchange their
+ * borders every few sweeps, in one cooperative launch that starts when the SMs have room for all of
+ * its tiles at once and takes those SMs whole; work of other streams runs on the other SMs, or after
+ * it.  (A depth, segment or layout in hs_config keeps the streaming passes, which share the SMs.)
+ * A tile's waits are bounded, a few seconds each.  One can only run out when another tile's block
+ * has stopped; hs_forward, hs_sweeps, hs_forward_noalloc, the batched calls and the training calls
+ * then leave NaN in the flow or the gradients that depend on it, although the call has returned
+ * HS_OK, and hs_wait_status reports it. */
+
+/* *device_status (a device int) receives HS_ERR_TIMEOUT if a bounded wait of any such launch on the
+ * current device has run out since the last hs_wait_status, else HS_OK, when `stream` reaches it.  No
+ * counterpart in the reference, whose runtime has no device-side waits. */
+HS_API hs_status hs_wait_status(int *device_status, void *stream);
+
 /* 2x2x2 derivatives in one pass: Ix = Dx*I0 + Dx*I1, Iy = Dy*I0 + Dy*I1,
  * It = Dt*I1 - Dt*I0 with Dx, Dy, Dt the 4-tap stencils over {0,1}^2 (weights -1/4,
  * +1/4 for Dx/Dy, 1/4 for Dt) and clamp-to-edge taps.  Bit-identical to the
@@ -313,6 +327,14 @@ HS_API hs_status hs_apply_hs_preconditioner(float s2, const float *diag0, const 
  * (1 .. 2^22, with a nanosleep back-off of at most 256 ns each) and writes HS_ERR_TIMEOUT to
  * *device_status (a device int the caller zeroed).  The kernel then returns normally. */
 HS_API hs_status hs_selftest_bounded_wait(int *device_status, int max_polls, void *stream);
+
+/* Self-test of the waits of the images held on the chip: hs_forward_train_batched and then
+ * hs_backward_batched with waits of max_polls polls (0 .. 2^22) instead of a few seconds.  At 0 polls
+ * tiles give up on one another: every wait ends, the kernels return, flow and gradients hold NaN and
+ * hs_wait_status reports HS_ERR_TIMEOUT. */
+HS_API hs_status hs_selftest_resident_wait(const hs_train_pair *pairs, int n, int iters, int ckpt_every,
+                                           void *workspace, size_t workspace_bytes,
+                                           const hs_config *cfg, int max_polls, void *stream);
 
 /* ---- Lucas-Kanade and Brox on the same grid substrate -------------------------- */
 

@@ -194,3 +194,69 @@ def test_batch_by_default_equals_per_pair_passes(cuda, name, fast):
     plan.capture()
     for _ in range(2):
         run(plan.replay)
+
+
+# ------------------------------------------------------------------ waits that run out
+
+def test_waits_that_run_out_leave_nan_and_a_status(cuda):
+    """Training on the chip with waits of 0 polls: tiles give up on one another, every wait ends, the
+    flow and the gradients say so, and the calls after it are right."""
+    import ctypes
+
+    lib = L.lib()
+    shapes = [(600, 799), (300, 402)]
+    cfg = L.make_config(fast_math=True)
+    planes = [images(s, 8, 40 + i) for i, s in enumerate(shapes)]
+    alpha, dalpha = torch.tensor([0.9], device="cuda"), torch.zeros(2, device="cuda")
+    arr = (L.hs_train_pair * 2)()
+    for i, (d, p) in enumerate(zip(arr, planes)):
+        d.I0, d.I1, d.u, d.v, d.dLdu, d.dLdv, d.dI0, d.dI1 = (t.data_ptr() for t in p)
+        d.alpha, d.dalpha = alpha.data_ptr(), dalpha.data_ptr() + 4 * i
+        d.H, d.W, d.ld = p[0].shape[0], p[0].shape[1], p[0].stride(0)
+    need = lib.hs_train_workspace_bytes(arr, 2, ITERS, CKPT)
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+
+    def run(polls):
+        L.check(lib.hs_selftest_resident_wait(arr, 2, ITERS, CKPT, D.ptr(ws), need, ctypes.byref(cfg), polls,
+                                              D.stream_handle()), "hs_selftest_resident_wait")
+        return [t.clone() for p in planes for t in (p[2], p[3], p[6], p[7])] + [dalpha.clone()]
+
+    D.check_waits()
+    ref = run(1 << 22)
+    D.check_waits()
+    assert all(torch.isfinite(t).all() for t in ref)
+    out = run(0)
+    with pytest.raises(L.HSError) as e:
+        D.check_waits()
+    assert e.value.status == L.HS_ERR_TIMEOUT
+    assert any(torch.isnan(t).any() for t in out[:4]) and torch.isnan(out[-1]).any()
+    D.check_waits()  # read once
+    for a, b in zip(run(1 << 22), ref):
+        equal(a, b, "the next call")
+    D.check_waits()
+
+
+def test_first_call_of_a_process_can_be_captured(cuda):
+    """hs_forward and the batched call set their kernels up inside a capture, too."""
+    import subprocess
+    import sys
+
+    code = """
+import torch
+from hindemith_b200 import _lib as L, device as D
+a, b, u, v = (t for t in D.empty_planes(4, 300, 402))
+a.copy_(torch.rand(300, 402)); b.copy_(torch.rand(300, 402))
+D.workspace(L.lib().hs_forward_workspace_bytes(300, 402, 404), a.device)
+s = torch.cuda.Stream()
+with torch.cuda.stream(s):
+    D.workspace(L.lib().hs_forward_workspace_bytes(300, 402, 404), a.device)
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g, stream=s):
+    D.hs_forward(a, b, 1.0, 30, out=(u, v))
+g.replay(); torch.cuda.synchronize()
+x, y = D.hs_forward(a, b, 1.0, 30)
+assert torch.equal(x, u) and torch.equal(y, v)
+print("captured")
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert "captured" in r.stdout, r.stderr[-2000:]

@@ -302,3 +302,24 @@ def test_training_cases_take_their_tile_heights(fake, fast):
             fake.reset()
             ls = train(fake, shapes, ITERS, CKPT, cfg=cfg, backward=back)
             assert [x.args[-1] for x in ls if x.kernel == name] == rows
+
+
+# ------------------------------------------------------------------ the wait status
+
+def test_wait_status_argument_checks():
+    lib = L.lib()
+    assert lib.hs_wait_status(None, None) == L.HS_ERR_INVALID_ARG
+    arr = train_pairs([(300, 402)])
+    need = lib.hs_train_workspace_bytes(arr, 1, 20, 5)
+    cfg = ctypes.byref(L.make_config())
+    assert lib.hs_selftest_resident_wait(arr, 1, 20, 5, P(WS), need, cfg, -1, None) == L.HS_ERR_INVALID_ARG
+    assert lib.hs_selftest_resident_wait(arr, 1, 20, 5, P(WS), need, cfg, (1 << 22) + 1, None) == L.HS_ERR_INVALID_ARG
+    assert lib.hs_selftest_resident_wait(arr, 1, 20, 5, P(WS), need - 1, cfg, 0, None) == L.HS_ERR_WORKSPACE
+    assert lib.hs_selftest_resident_wait(arr, 1, 20, 5, P(WS + 16), need, cfg, 0, None) == L.HS_ERR_ALIGNMENT
+    arr[0].dLdu = None
+    assert lib.hs_selftest_resident_wait(arr, 1, 20, 5, P(WS), need, cfg, 0, None) == L.HS_ERR_INVALID_ARG
+
+
+def test_wait_status_asks_both_directions(fake):
+    assert fake.lib.hs_wait_status(P(1 << 36), None) == L.HS_OK
+    assert [x.first for x in fake.launches()] == [1 << 36] * 2

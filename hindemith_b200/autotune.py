@@ -36,9 +36,10 @@ def _key(dev_name, H, W, ld, fast_math):
 DEFAULT_TUNING_SWEEPS = 240
 
 
-def _sweep_key(dev_name, H, W, ld, fast_math, sweeps):
-    """Cache key of a sweep tuning; a run over another sweep count is cached apart."""
-    key = _key(dev_name, H, W, ld, fast_math) + "|layout"
+def _sweep_key(dev_name, H, W, ld, fast_math, sweeps, passes_only=False):
+    """Cache key of a sweep tuning; a run over another sweep count, and one among the passes only,
+    are cached apart."""
+    key = _key(dev_name, H, W, ld, fast_math) + "|layout" + ("|passes" if passes_only else "")
     return key if sweeps == DEFAULT_TUNING_SWEEPS else key + f"|s{sweeps}"
 
 
@@ -89,18 +90,20 @@ def time_config(Ix, Iy, It, u, v, T, seg, fast_math, sweeps, reps=5, layout=0):
 
 def best_sweep_config(H: int, W: int, ld: int, fast_math: bool = True,
                       candidates=T_CANDIDATES,
-                      sweeps: int = DEFAULT_TUNING_SWEEPS) -> Tuple[int, int, int]:
+                      sweeps: int = DEFAULT_TUNING_SWEEPS,
+                      passes_only: bool = False) -> Tuple[int, int, int]:
     """(sweeps_per_pass, rows_per_segment, layout) fastest on the current device for HxW;
     both layouts (2 and 4 columns per lane) compete in the fast form, and (0, 0, 0), the
     library's own choice, which holds an image that fits the chip there for all sweeps.  Every
-    candidate is timed over `sweeps` sweeps: pass the workload's own count when it is known (the last, partial
-    pass differs by depth)."""
+    candidate is timed over `sweeps` sweeps: pass the workload's own count when it is known (the
+    last, partial pass differs by depth).  passes_only leaves (0, 0, 0) out, for a caller that adds
+    a segment of its own to the answer: with one the library runs the passes."""
     import torch
 
     from . import device as D
 
     dev_name = torch.cuda.get_device_name()
-    key = _sweep_key(dev_name, H, W, ld, fast_math, sweeps)
+    key = _sweep_key(dev_name, H, W, ld, fast_math, sweeps, passes_only)
     with _lock:
         if not _cache:
             _load_file()
@@ -120,7 +123,8 @@ def best_sweep_config(H: int, W: int, ld: int, fast_math: bool = True,
             for seg in _seg_candidates(H, W, T):
                 ms = time_config(Ix, Iy, It, u, v, T, seg, fast_math, sweeps, layout=layout)
                 results.append((ms, T, seg, layout))
-    results.append((time_config(Ix, Iy, It, u, v, 0, 0, fast_math, sweeps), 0, 0, 0))
+    if not passes_only:
+        results.append((time_config(Ix, Iy, It, u, v, 0, 0, fast_math, sweeps), 0, 0, 0))
     results.sort()
     best = tuple(results[0][1:])
     log = os.environ.get("HS_AUTOTUNE_LOG")

@@ -706,7 +706,8 @@ class Executor:
             from .autotune import best_sweep_config
 
             T, seg, layout = best_sweep_config(Ix.shape[0], Ix.shape[1], Ix.stride(0),
-                                               fast_math=bool(cfg.fast_math))
+                                               fast_math=bool(cfg.fast_math),
+                                               passes_only=cfg.rows_per_segment > 0)
             cfg.sweeps_per_pass, cfg.layout = T, layout
             if cfg.rows_per_segment == 0:
                 cfg.rows_per_segment = seg

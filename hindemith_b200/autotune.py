@@ -47,23 +47,37 @@ def _file():
     return os.environ.get("HS_AUTOTUNE_CACHE")
 
 
-def _load_file():
+# What an answer was chosen from.  In the file a key carries it: the answer of a tuning that did not
+# time the library's own choice is not this one's, which would keep an image that fits the chip in
+# the passes (1080p: 526 against 841 Gpix-it/s), and stays in the file for the program that made it.
+_CANDIDATES = "|+own choice"
+
+
+def _read_file() -> dict:
     path = _file()
     if path and os.path.exists(path):
         try:
             with open(path) as f:
-                for k, v in json.load(f).items():
-                    _cache.setdefault(k, tuple(v))
-        except (OSError, ValueError):
+                return dict(json.load(f))
+        except (OSError, ValueError, TypeError):
             pass
+    return {}
+
+
+def _load_file():
+    for k, v in _read_file().items():
+        if k.endswith(_CANDIDATES):
+            _cache.setdefault(k[:-len(_CANDIDATES)], tuple(v))
 
 
 def _save_file():
     path = _file()
     if path:
+        entries = _read_file()
+        entries.update({k + _CANDIDATES: list(v) for k, v in _cache.items()})
         try:
             with open(path, "w") as f:
-                json.dump({k: list(v) for k, v in _cache.items()}, f, indent=1)
+                json.dump(entries, f, indent=1)
         except OSError:
             pass
 

@@ -36,3 +36,27 @@ def test_a_tuning_among_the_passes_is_cached_apart():
     b = autotune._sweep_key("B200", 480, 640, 640, True, autotune.DEFAULT_TUNING_SWEEPS, True)
     c = autotune._sweep_key("B200", 480, 640, 640, True, 77, True)
     assert len({a, b, c}) == 3
+
+
+def test_a_cache_file_keeps_apart_what_answers_were_chosen_from(monkeypatch, tmp_path):
+    """Answers from before the library's own choice was timed are not taken for this tuner's, and
+    stay in the file; its own are read back."""
+    import json
+
+    path = tmp_path / "cache.json"
+    key = autotune._sweep_key("B200", 1080, 1920, 1920, True, 500)
+    path.write_text(json.dumps({key: [7, 0, 2]}))
+    monkeypatch.setenv("HS_AUTOTUNE_CACHE", str(path))
+    monkeypatch.setattr(autotune, "_cache", {})
+    autotune._load_file()
+    assert key not in autotune._cache
+    autotune._cache[key] = (0, 0, 0)
+    autotune._save_file()
+    monkeypatch.setattr(autotune, "_cache", {})
+    autotune._load_file()
+    assert autotune._cache == {key: (0, 0, 0)}
+    assert json.loads(path.read_text())[key] == [7, 0, 2]
+    path.write_text("not json")
+    autotune._load_file()
+    autotune._save_file()
+    assert list(json.loads(path.read_text()).values()) == [[0, 0, 0]]

@@ -60,3 +60,27 @@ def test_a_cache_file_keeps_apart_what_answers_were_chosen_from(monkeypatch, tmp
     autotune._load_file()
     autotune._save_file()
     assert list(json.loads(path.read_text()).values()) == [[0, 0, 0]]
+
+
+def test_every_candidate_is_warmed_up(monkeypatch):
+    """The call before the timed ones launches the candidate's kernel: at depth 0 too."""
+    class Event:
+        def __init__(self, enable_timing):
+            pass
+
+        def record(self):
+            pass
+
+        def synchronize(self):
+            pass
+
+        def elapsed_time(self, other):
+            return 1.0
+
+    calls = []
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    monkeypatch.setattr(device, "hs_sweeps", lambda *a: calls.append((a[4], a[-1].sweeps_per_pass)))
+    for T in (0, 1, 4, 7):
+        calls.clear()
+        autotune.time_config(*[None] * 5, T, 0, True, 240, reps=2)
+        assert calls == [(max(T, 2), T), (240, T), (240, T)]

@@ -31,7 +31,9 @@ sys.path.insert(0, HERE)
 
 METRIC = "HS Mpix-iters/s fwd and fwd+bwd (batched vs plain) on 1 B200; % HBM roofline"
 UNIT = "Mpix-iters/s"
-BYTES_PER_PX_PASS = 28  # read Ix, Iy, It, u, v; write u, v (FP32)
+BYTES_PER_PX_PASS = 28  # a pass: read Ix, Iy, It, u, v; write u, v (FP32)
+BYTES_PER_PX_CHIP = 16  # an image on the chip: read I0, I1; write u, v, once for all sweeps
+LANE_OPS_FAST, LANE_OPS_EXACT = 15, 36  # FP32 lane operations of a pixel's sweep
 L2_FLUSH_BYTES = 256 << 20
 
 
@@ -382,6 +384,21 @@ def timed_events(fn, k, warmup, flush, stream, label):
     return sum(a.elapsed_time(b) for a, b in evs) / 1e3
 
 
+def sweep_launches(lib, H, W, ld, iters, cfg):
+    """How hs_forward runs the sweeps of such a pair: (launches, kernel, whether it stays on the chip)."""
+    import ctypes
+
+    n = lib.hs_sweeps_per_launch(H, W, ld, iters, ctypes.byref(cfg))
+    if n > 8:  # (no pass is deeper)
+        return 1, "hs_resident_kernel", True
+    if cfg.fast_math and (cfg.layout == 2 or (cfg.layout == 0 and H * W >= 250_000)):
+        # 4 columns per lane; the ring is in tensor memory from 3.3 Mpx up (kTmPixels, hs_sweep.cu)
+        kernel = f"hs_stream_{'tm' if H * W >= 3_300_000 else 'w'}_kernel<{n}>"
+    else:  # the main loop is unrolled at depths 1 and 2
+        kernel = f"hs_stream_kernel<{n},{'true' if cfg.fast_math else 'false'},{'true' if n <= 2 else 'false'}>"
+    return -(-iters // n), kernel, False
+
+
 def measure_batched(args, rank, flush, peak, checks=None):
     """The mixed batch (64 pairs, 320x240 .. 2048x2048, alpha in [0.5, 2], 100/200/500
     sweeps): one graph-captured persistent launch, against one plain hs_forward per pair."""
@@ -429,10 +446,11 @@ def measure_batched(args, rank, flush, peak, checks=None):
     same = all(torch.equal(plan.u[i], outs[i][0]) and torch.equal(plan.v[i], outs[i][1])
                for i in range(len(specs)))
     px_it = plan.pixel_iters
-    # T = 0: an image that fits the chip moves its planes once, a larger one once per 7 sweeps
-    passes = sum(sp.H * sp.W * ((sp.iters + T - 1) // T if T else
-                                1 if sp.H * sp.W < 2_100_000 else (sp.iters + 6) // 7) for sp in specs)
-    achieved = BYTES_PER_PX_PASS * passes * args.steps / t_b / 1e9
+    moved = 0
+    for i, sp in enumerate(specs):
+        launches, _, chip = sweep_launches(L.lib(), sp.H, sp.W, D.ld_of(plan.I0[i]), sp.iters, cfg)
+        moved += sp.H * sp.W * (BYTES_PER_PX_CHIP if chip else BYTES_PER_PX_PASS * launches)
+    achieved = moved * args.steps / t_b / 1e9
 
     # the same batch at depth 4, where a pass is closer to HBM-bound than issue-bound
     cfg3 = L.make_config(sweeps_per_pass=4, rows_per_segment=96, fast_math=not args.exact,
@@ -979,10 +997,7 @@ def main():
         T, seg, layout = autotune.best_sweep_config(H, W, ld, fast_math=not args.exact, sweeps=iters)
     cfg = L.make_config(sweeps_per_pass=T, rows_per_segment=seg, fast_math=not args.exact,
                         layout=layout)
-    # the layout the library runs (hs_config.layout 0 chooses by image size)
-    wide = (not args.exact) and (layout == 2 or (layout == 0 and H * W >= 2_000_000))
-    # T = 0: the library holds the image on the chip for all sweeps (one launch)
-    passes = (iters + T - 1) // T if T else 1
+    passes, kernel, chip = sweep_launches(L.lib(), H, W, ld, iters, cfg)
     flush = torch.empty(L2_FLUSH_BYTES // 4, dtype=torch.float32, device="cuda")
 
     uv = D.empty_planes(2, H, W)
@@ -1094,13 +1109,10 @@ def main():
     value = job_rate(H * W * iters * args.steps, world, t_step) / 1e6
     e2e_value = job_rate(H * W * iters * args.steps, world, t_e2e) / 1e6
     peak, peak_kind = load_peaks()
-    launch_s = t_sweeps / (args.steps * passes)
-    achieved = BYTES_PER_PX_PASS * H * W / launch_s / 1e9
-    # the wide layout's ring is in tensor memory from 3.3 Mpx up (kTmPixels in hs_sweep.cu); the
-    # 2-column kernel's main loop is unrolled at depths 1 and 2
-    kernel = (f"hs_stream_{'tm' if H * W >= 3300000 else 'w'}_kernel<{T}>" if wide else
-              f"hs_stream_kernel<{T},{'false' if args.exact else 'true'},"
-              f"{'true' if T <= 2 else 'false'}>") if T else "hs_resident_kernel"
+    # on the chip the step is the one launch (derivatives in it); else the passes alone
+    launch_s = (t_step if chip else t_sweeps) / (args.steps * passes)
+    px_bytes = BYTES_PER_PX_CHIP if chip else BYTES_PER_PX_PASS
+    achieved = px_bytes * H * W / launch_s / 1e9
     # ncu figures of this very kernel at this shape (profiles/), when one was captured
     traffic, prof = None, {}
     tpath = os.path.join(HERE, "profiles", "sweep_traffic.json")
@@ -1110,8 +1122,10 @@ def main():
         traffic = prof.get("dram_bytes")
     # issue slots the launch used: its warp instructions over the SMSPs' slots in its time
     sm_mhz = clocks.get("sm_mhz") or 1965.0
-    issue_frac = (prof["inst"] / (launch_s * torch.cuda.get_device_properties(0).multi_processor_count
-                                  * 4 * sm_mhz * 1e6) if "inst" in prof else None)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    lane_ops = LANE_OPS_EXACT if args.exact else LANE_OPS_FAST
+    lane_peak = sms * 128 * sm_mhz * 1e6
+    issue_frac = (prof["inst"] / (launch_s * sms * 4 * sm_mhz * 1e6) if "inst" in prof else None)
 
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -1120,17 +1134,23 @@ def main():
         "data": "synthetic (seeded blurred noise + sinusoidal flow; see hindemith_b200/synthetic.py)",
         "config": headline_config(workload, H, W, iters, alpha, world),
         "tuning": {"sweeps_per_pass": T, "rows_per_segment": seg,
-                   "columns_per_lane": 4 if wide or not T else 2, "fast_math": not args.exact,
+                   "columns_per_lane": 2 if kernel.startswith("hs_stream_kernel") else 4,
+                   "on_chip": chip, "fast_math": not args.exact,
                    "autotuned": args.sweeps_per_pass == 0},
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "traffic": traffic,
-                     "kernel": kernel, "peak_source": peak_kind,
-                     "bytes_per_launch": BYTES_PER_PX_PASS * H * W,
+        "roofline": ({"bound": "fp32", "achieved": lane_ops * H * W * iters / launch_s / 1e9,
+                      "peak": lane_peak / 1e9, "unit": "G lane-ops/s",
+                      "frac": lane_ops * H * W * iters / launch_s / lane_peak,
+                      "peak_source": "SMs x 128 FP32 lanes x the sampled SM clock",
+                      "lane_ops_per_px_sweep": lane_ops} if chip else
+                     {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                      "frac": achieved / peak, "peak_source": peak_kind}) |
+                    {"kernel": kernel, "hbm_gbs": achieved, "hbm_frac": achieved / peak,
+                     "bytes_per_launch": px_bytes * H * W, "traffic": traffic,
                      "avg_launch_us": launch_s * 1e6,
                      "traffic_source": prof.get("summary"),
                      "issue_slot_frac": issue_frac,
-                     "note": ("the image stays on the chip for all sweeps (one launch): bound by the "
-                              "FP32 pipe and its register reads, not by HBM") if not T else
+                     "note": ("the image stays on the chip for all sweeps, one launch: what it moves "
+                              "is its images and its flow, once") if chip else
                              "at 1920x1080 the pair's 41.5 MB working set is L2-resident within "
                              "a step: the kernel is issue/latency-bound, so issue_slot_frac (the "
                              "profiled warp instructions per launch over 4 issue slots x SMs x "
@@ -1149,7 +1169,7 @@ def main():
                        {"value": H * W * iters * max(1, args.steps // 2) / t_exact / 1e6,
                         "unit": UNIT, "sweeps_per_pass": Te, "rows_per_segment": sege,
                         "note": "bit-identical to the reference's FP32 semantics"}),
-        "gpu_launches": (1 + passes if T else 1) * args.steps,  # (T = 0: derivatives included)
+        "gpu_launches": (1 if chip else 1 + passes) * args.steps,  # (on the chip: derivatives included)
         "clocks": clocks,
     }
     # the batched and differentiable workloads are single-GPU measurements

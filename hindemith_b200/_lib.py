@@ -133,6 +133,7 @@ SIGNATURES = {
     "hs_apply_hs_preconditioner": (_i, [_f, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _vp]),
     "hs_selftest_bounded_wait": (_i, [_vp, _i, _vp]),
     "hs_wait_status": (_i, [_vp, _vp]),
+    "hs_sweeps_per_launch": (_i, [_i, _i, _i, _i, _cfgp]),
     "hs_selftest_resident_wait": (_i, [_vp, _i, _i, _i, _vp, _sz, _cfgp, _i, _vp]),
     "hs_lk_least_squares": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp, _vp]),
     "hs_set_brox_matrix": (_i, [_vp, _i, _i, _i, _f, _vp, _sz, _i, _vp, _vp]),

@@ -399,6 +399,15 @@ size_t hs_forward_workspace_bytes(int H, int W, int ld) {
     return 5 * round_up(plane_bytes(H, ld), 256);
 }
 
+int hs_sweeps_per_launch(int H, int W, int ld, int iters, const hs_config *cfg) {
+    clear_error();
+    ResolvedConfig rc;
+    if (check_plane_geometry(H, W, ld) != HS_OK || resolve_config(cfg, &rc) != HS_OK || iters < 0) return 0;
+    apply_shape_default(rc, H, W);
+    ResidentPlan pl;
+    return wants_resident(rc) && resident_plan(H, W, iters, hs_forward_workspace_bytes(H, W, ld), pl) ? iters : rc.T;
+}
+
 hs_status hs_sweeps(const float *Ix, const float *Iy, const float *It, int H, int W, int ld,
                     float alpha2, int iters, float *u, float *v, void *workspace,
                     size_t workspace_bytes, const hs_config *cfg, void *stream) {

@@ -145,6 +145,10 @@ HS_API hs_status hs_sweeps(const float *Ix, const float *Iy, const float *It, in
 /* Scratch needed by hs_forward: five planes (Ix, Iy, It and the ping-pong copy). */
 HS_API size_t hs_forward_workspace_bytes(int H, int W, int ld);
 
+/* Sweeps that hs_forward runs per launch for such a pair: `iters` for an image held on the chip, else
+ * the depth of its passes (1..8); 0 for invalid arguments.  Host-only. */
+HS_API int hs_sweeps_per_launch(int H, int W, int ld, int iters, const hs_config *cfg);
+
 /* The plain per-pair drop-in: derivatives, u = v = 0, `iters` sweeps with
  * alpha2 = alpha * alpha (FP32).  Replaces backend.run for a compiled Horn-Schunck
  * program (backend.cpp:320-638) end to end on the device. */

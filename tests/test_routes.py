@@ -323,3 +323,37 @@ def test_wait_status_argument_checks():
 def test_wait_status_asks_both_directions(fake):
     assert fake.lib.hs_wait_status(P(1 << 36), None) == L.HS_OK
     assert [x.first for x in fake.launches()] == [1 << 36] * 2
+
+
+# ------------------------------------------------------------------ what the benchmark reports
+
+@pytest.mark.parametrize("H,W", [(16, 16), (240, 320), (480, 640), (1080, 1920), (1100, 1925), (2048, 2048), (3, 3000), (20000, 60)])
+@pytest.mark.parametrize("fast", [True, False])
+@pytest.mark.parametrize("T,layout", [(0, 0), (0, 1), (3, 0), (5, 1), (7, 2)])
+def test_benchmark_names_the_launches_of_its_step(fake, H, W, fast, T, layout):
+    """Launches, kernel and depth as hs_forward makes them, at every size and with every tuning."""
+    import bench
+
+    if layout == 2 and not fast:
+        pytest.skip("the exact form has 2 columns per lane")
+    cfg = L.make_config(sweeps_per_pass=T, fast_math=fast, layout=layout)
+    ls = forward(fake, H, W, 500, A, B, C, D, cfg)
+    launches, kernel, chip = bench.sweep_launches(fake.lib, H, W, pad(W), 500, cfg)
+    sweeps = [x for x in ls if x.kernel.startswith(("hs_resident", "hs_stream"))]
+    assert (len(sweeps), chip) == (launches, sweeps[0].kernel == "hs_resident_kernel")
+    if chip:
+        assert len(ls) == 1 and kernel == "hs_resident_kernel"
+    else:
+        args = ",".join([str(sweeps[0].args[0])] + ["true" if a else "false" for a in sweeps[0].args[1:]])
+        assert kernel == f"{sweeps[0].kernel}<{args}>"
+
+
+def test_sweeps_per_launch_argument_checks():
+    q = L.lib().hs_sweeps_per_launch
+    cfg = L.make_config()
+    assert q(0, 8, 8, 5, ctypes.byref(cfg)) == 0
+    assert q(8, 8, 6, 5, ctypes.byref(cfg)) == 0
+    assert q(8, 8, 8, -1, ctypes.byref(cfg)) == 0
+    assert q(8, 8, 8, 5, ctypes.byref(L.make_config(sweeps_per_pass=9))) == 0
+    assert q(8, 8, 8, 1, ctypes.byref(cfg)) == 4
+    assert q(8, 8, 8, 50, ctypes.byref(L.make_config(sweeps_per_pass=3))) == 3

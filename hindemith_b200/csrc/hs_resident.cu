@@ -3,14 +3,16 @@
 //
 // Measured on one B200 (hs_forward, us per call, streaming passes at their default depth ->
 // resident):
-//   1920x1080 x 500 sweeps, fast   2003 -> 1244      1901x1037 x 200, exact  1464 -> 958
-//   320x240 x 100, fast             171 ->  112       640x480 x 200, exact    855 -> 317
+//   1920x1080 x 500 sweeps, fast   2002 -> 1240      1901x1037 x 200, exact  1465 -> 945
+//   320x240 x 100, fast             170 ->  108       640x480 x 200, exact    858 -> 312
 // Bound (1080p, fast, 16 x 8 rows): of 2.4 us per sweep, 1.7 us are the sweep itself (the FP32
 // pipe and the register reads of its packed operations: fma.rn.f32x2 with three distinct
 // operands issues every 3.1 clocks, with a shared one every 2.2) and 0.7 us the exchange's share
 // (a quarter of 2.8 us: shared-memory staging and one round trip to L2).  16 warps of 128
 // registers run it faster than 8 of 255 (1.72 against 2.14 us per sweep): the state of R = 16
-// rows leaves too few warps to cover the shuffles.
+// rows leaves too few warps to cover the shuffles.  The 128 registers do not hold all: at R = 8 the
+// fast form spills 120 B of stores and 276 of loads per thread, the exact one 436 and 672; up to
+// R = 4 the fast form spills nothing.
 #include <algorithm>
 #include <cstring>
 #include <mutex>

@@ -128,7 +128,8 @@ HS_API hs_status hs_wait_status(int *device_status, void *stream);
 HS_API hs_status hs_derivs(const float *I0, const float *I1, int H, int W, int ld, float *Ix,
                     float *Iy, float *It, void *stream);
 
-/* Scratch needed by hs_sweeps: two planes (the ping-pong copy of u, v). */
+/* Scratch needed by hs_sweeps: two planes (the ping-pong copy of u, v).  A larger workspace may be used
+ * for lower tiles of an image held on the chip; the results are the same. */
 HS_API size_t hs_sweeps_workspace_bytes(int H, int W, int ld);
 
 /* `iters` Jacobi sweeps in place on (u, v), from their current contents:
